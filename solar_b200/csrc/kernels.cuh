@@ -420,8 +420,9 @@ enum { mD = 0, mXYD, mC, mXYC, mDivX, mDivY, mTX, mTY, mVol, mCount };
 //   lead ring (kLead slots): the p tile with a 3-point halo and the v_r tile of plane m.
 //     Plane m is needed from iteration m-3 (own values enter the 7-deep radial register
 //     windows of p and v_r) until iteration m (xi/eta derivatives of p).
-//   tile ring (kTile slots): v_xi with its xi halo, v_eta with its eta halo, rho and the
-//     RK registers qw of plane k, needed at iteration k only.
+//   tile ring (kTile slots): v_xi with its xi halo, v_eta with its eta halo, rho, the
+//     RK registers qw, the radial coefficients and (over a 3-D sound speed) c^2 of plane k,
+//     needed at iteration k only.
 // Thread 0 refills a slot right after the CTA barrier that closes the iteration using it,
 // so up to kLead-4 lead planes and kTile-1 tile planes are in flight while a plane is
 // computed.  The radial window is clamped at the two ends of the shell, where the
@@ -442,9 +443,10 @@ struct StageArgs {
   CUtensorMap mY;           // input buffer, box TX x (TY+6)
   CUtensorMap mO;           // input buffer, box TX x TY
   CUtensorMap mW;           // qw buffer,    box TX x TY
+  CUtensorMap mC2;          // compact c^2,  box TX x TY (only with c2)
   T* qout;
   T* qw;
-  const T* rad;             // [kNumRadial][nr]
+  const T* radT;            // [nr][16]: the radial rows of a plane together
   const T* met;             // [kNumMetric][n][n]
   const T* c2;              // optional compact c^2 [face][k][j][i] (run-shared) or nullptr
   T* divout;                // MODE 4/5: compact divergence [face][k][j][i]
@@ -499,10 +501,16 @@ struct StageLayout {
   static constexpr size_t Y_BYTES = align128(YB * sizeof(T));
   static constexpr size_t O_BYTES = align128(OB * sizeof(T));
   static constexpr size_t LEAD = P_BYTES + O_BYTES;                    // p box + v_r
-  static constexpr size_t TILE = X_BYTES + Y_BYTES + NO * O_BYTES;     // v_xi, v_eta, (rho), qw
+  static constexpr size_t RAD = X_BYTES + Y_BYTES + NO * O_BYTES;      // v_xi, v_eta, (rho), qw, then
+  static constexpr size_t TILE = RAD + align128(16 * sizeof(T));       // the row of radial coefficients
   static constexpr int RING = TileRing<T>::value;
   static constexpr size_t BAR = kLead * LEAD + RING * TILE;
   static constexpr size_t TOTAL = BAR + (kLead + RING) * sizeof(uint64_t);
+  // over a 3-D sound speed the launch adds one c^2 box per tile slot after the rings (with a
+  // radial c^2 that memory stays free: it decides between three and four CTAs per SM for the
+  // 32 x 8 float tile with rho)
+  static constexpr size_t C2 = align128(TOTAL);
+  static constexpr size_t TOTAL_C2 = C2 + RING * O_BYTES;
 };
 
 // Each thread owns V consecutive points of one row (V = 16 bytes / sizeof(T)), so the
@@ -539,6 +547,10 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
   auto clampk = [nr](int k) { return min(max(k - 3, 0), nr - 7); };
   const int m_lo = clampk(kb), m_hi = clampk(ke - 1) + 6;
 
+  // c^2 of a 3-D sound speed comes through the ring with its plane: loaded from global memory
+  // at its use it stalled every plane (a stage at 6 x 160^2 x 96 in double 574 us, now 427; at
+  // 6 x 96^3 219 -> 164 us in double, 100 -> 75 in float).
+  const bool tc2 = MODE != 3 && a.c2 != nullptr;
   auto lead = [&](int slot) { return smem + slot * L::LEAD; };
   auto tile = [&](int slot) { return smem + kLead * L::LEAD + slot * L::TILE; };
   const int xP = IOFF + i0 - 4, yP = JOFF + j0 - 3;   // p / v_xi boxes start 4 columns left
@@ -554,8 +566,10 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
     uint32_t bytes = (L::XB + L::YB) * sizeof(T);
     if (HAS_RHO && MODE != 3) bytes += L::OB * sizeof(T);
     if (MODE == 0) bytes += g.nf * L::OB * sizeof(T);
-    mbar_expect_tx(b, bytes);
+    if (tc2) bytes += L::OB * sizeof(T);
+    mbar_expect_tx(b, bytes + 16 * sizeof(T));
     unsigned char* t = tile(slot);
+    if (tc2) tma_load_3d(smem + L::C2 + slot * L::O_BYTES, &a.mC2, i0, j0, face * nr + k, b);
     tma_load_3d(t, &a.mX, xP, yO, (zbase + sX) * nr + k, b);
     tma_load_3d(t + L::X_BYTES, &a.mY, xO, yP, (zbase + sY) * nr + k, b);
     if (HAS_RHO && MODE != 3)
@@ -563,6 +577,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
     if (MODE == 0)
       for (int s = 0; s < g.nf; ++s)
         tma_load_3d(t + L::X_BYTES + L::Y_BYTES + (QOFF + s) * L::O_BYTES, &a.mW, xO, yO, (zbase + s) * nr + k, b);
+    bulk_load(t + L::RAD, a.radT + (size_t)k * 16, 16 * sizeof(T), b);
   };
 
   // per-point constants (constant tables: read before the dependency wait)
@@ -615,24 +630,6 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
   const int yc = (ty + 3) * TX + V * cx;
   const int oc = ty * TX + V * cx;
 
-  // radial coefficients of the current plane; the next plane's are loaded one iteration
-  // ahead so their latency hides behind the compute
-  struct Rad { T facr, invr, rho0, inv_rho0, c2rho0, rho0g0, sig, drho0, g0rho0, frc; };
-  auto load_rad = [&](int k) {
-    Rad r;
-    r.frc = FORCE ? __ldg(a.force_r + k) : T(0);
-    r.facr = __ldg(a.rad + rFacR * nr + k);
-    r.invr = __ldg(a.rad + rInvR * nr + k);
-    r.rho0 = __ldg(a.rad + rRho0 * nr + k);
-    r.inv_rho0 = __ldg(a.rad + rInvRho0 * nr + k);
-    r.c2rho0 = __ldg(a.rad + rC2Rho0 * nr + k);
-    r.rho0g0 = __ldg(a.rad + rRho0G0 * nr + k);
-    r.sig = __ldg(a.rad + rSigma * nr + k);
-    r.drho0 = HAS_RHO ? __ldg(a.rad + rDRho0 * nr + k) : T(0);
-    r.g0rho0 = HAS_RHO ? __ldg(a.rad + rG0Rho0 * nr + k) : T(0);
-    return r;
-  };
-  Rad rc = load_rad(kb);
   T pw[7][V], vw[7][V];
 #pragma unroll
   for (int s = 0; s < 7; ++s)
@@ -661,7 +658,6 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
       if (++slot_q == kLead) { slot_q = 0; phase_q ^= 1; }
     }
     if (ok && !mbar_wait(&barT[slot_t], phase_t, a.wc, kErrStageTile)) { ok = false; tile_fail = true; }
-    const Rad rn = load_rad(min(k + 1, nr - 1));
     const T* sp = reinterpret_cast<const T*>(lead(slot_k));
     const unsigned char* tb = tile(slot_t);
     const T* sx = reinterpret_cast<const T*>(tb);
@@ -688,8 +684,18 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
           const int sl = HAS_RHO ? f : f - 1;
           ldv(reinterpret_cast<const T*>(tb + L::X_BYTES + L::Y_BYTES + (QOFF + sl) * L::O_BYTES) + oc, qwv[f]);
         }
-    const T facr = rc.facr;
-    const T invr = rc.invr;
+    const T* sc2 = reinterpret_cast<const T*>(smem + L::C2 + slot_t * L::O_BYTES) + oc;
+    // The plane's radial coefficients come with its ring slot, every thread reading the same
+    // words with 16-byte loads.  Loaded from global memory one plane ahead they cost 9 loads per
+    // thread and plane and 36 registers in double, which spilled with a source term (a forced
+    // stage at 6 x 80^2 x 50 in double 93 -> 74 us; 6 x 192^2 x 120 in float 332 -> 313, 6 x
+    // 128^3 in float 149.2 -> 146.6; read word by word at their uses 150).
+    T rr[12];
+#pragma unroll
+    for (int m = 0; m < 12; m += V) ldv(reinterpret_cast<const T*>(tb + L::RAD) + m, rr + m);
+    const T facr = rr[rFacR], invr = rr[rInvR];
+    T frc = T(0);
+    if (FORCE) frc = __ldg(a.force_r + k);
     const bool interior = k >= 3 && k <= nr - 4;
     const int offk = k - ks;
     const int brow = k < 3 ? k : nr - 1 - k;
@@ -730,18 +736,17 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
       if (MODE == 3) {
         o0[q] = gxi; o1[q] = geta; o2[q] = dpr; o3[q] = div;
       } else {
-        const T rho0 = rc.rho0, inv_rho0 = rc.inv_rho0;
-        T c2rho0 = rc.c2rho0;
-        if (a.c2) c2rho0 = a.c2[((long long)face * nr + k) * P2 + p2 + q] * rho0;
+        const T rho0 = rr[rRho0], inv_rho0 = rr[rInvRho0];
+        const T c2rho0 = tc2 ? sc2[q] * rho0 : rr[rC2Rho0];
         r_vx[q] = -gxi * inv_rho0;
         r_ve[q] = -geta * inv_rho0;
         r_vr[q] = -dpr * inv_rho0;
-        r_p[q] = -c2rho0 * div + rc.rho0g0 * v_r;
+        r_p[q] = -c2rho0 * div + rr[rRho0G0] * v_r;
         if (HAS_RHO) {
-          r_rho[q] = -rho0 * div - v_r * rc.drho0;
-          r_vr[q] -= rho[q] * rc.g0rho0;
+          r_rho[q] = -rho0 * div - v_r * rr[rDRho0];
+          r_vr[q] -= rho[q] * rr[rG0Rho0];
         }
-        if (FORCE) r_vr[q] += f_xy[q] * rc.frc;         // + S(theta, phi, t) e_r
+        if (FORCE) r_vr[q] += f_xy[q] * frc;         // + S(theta, phi, t) e_r
       }
     }
     const long long kp = (long long)k * g.plane;
@@ -760,7 +765,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
     } else {
       // BC_RHS (bc_acoustic_wave.f90:14-34) then SPONGE (sponge.f90:40-50)
       const bool bc = (k == 0 || k == nr - 1);
-      const T sig = rc.sig;
+      const T sig = rr[rSigma];
       const T dt = a.dt, alpha = a.alpha, beta = a.beta;
       // qw = alpha qw + dt rhs ; q = q + beta qw   (timestep.f90:68-69)
       auto update = [&](int f, const T* qv, const T* rv, bool damped) {
@@ -792,7 +797,6 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
     }
     if (++slot_t == kTile) { slot_t = 0; phase_t ^= 1; }
     if (++slot_k == kLead) slot_k = 0;
-    rc = rn;
   }
   if (failed && tid == 0 && loads) {
     // at the break in iteration k: tile planes [kb, min(k + kTile, ke)) were issued and

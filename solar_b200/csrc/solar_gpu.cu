@@ -424,19 +424,21 @@ static int launch_stage_t(solar_ctx* c, StageArgs<T>& a, const void* qin) {
   using L = StageLayout<T, TX, TY, HAS_RHO>;
   if (!make_map(c, qin, TX + 8, TY + 6, &a.mP) || !make_map(c, qin, TX + 8, TY, &a.mX) ||
       !make_map(c, qin, TX, TY + 6, &a.mY) || !make_map(c, qin, TX, TY, &a.mO) ||
-      !make_map(c, c->W, TX, TY, &a.mW))
+      !make_map(c, c->W, TX, TY, &a.mW) || (a.c2 && !make_compact_map(c, a.c2, TX, TY, &a.mC2)))
     return fail(SOLAR_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   static bool attr_set = false;
   if (!attr_set) {
     CK(cudaFuncSetAttribute(stage_kernel<T, TX, TY, MODE, HAS_RHO, FORCE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)L::TOTAL));
+                            (int)L::TOTAL_C2));
     attr_set = true;
   }
+  const size_t smem = a.c2 ? L::TOTAL_C2 : L::TOTAL;
+  if (!a.c2) a.mC2 = a.mO;                         // unused
   const int nchunks = (c->g.k1 - c->g.k0 + a.kchunk - 1) / a.kchunk;
   const int ntiles = stage_tile_count(a.tsel, c->g.n / TX, c->g.n / TY);
   if (ntiles <= 0) return SOLAR_OK;                // no interior tiles at this size
   dim3 grid(ntiles, nchunks, launched_runs(c, a.runs) * c->g.nface);
-  CK(launch_pdl(stage_kernel<T, TX, TY, MODE, HAS_RHO, FORCE>, grid, dim3(TX / Vec16<T>::V, TY), L::TOTAL, c->stream, a));
+  CK(launch_pdl(stage_kernel<T, TX, TY, MODE, HAS_RHO, FORCE>, grid, dim3(TX / Vec16<T>::V, TY), smem, c->stream, a));
   return SOLAR_OK;
 }
 
@@ -483,7 +485,7 @@ static int launch_stage(solar_ctx* c, const void* qin, void* qout, int mode, int
   a.force_r = forced ? (const T*)c->force_r : nullptr;
   a.qout = (T*)qout;
   a.qw = (T*)c->W;
-  a.rad = (const T*)c->dt.rad;
+  a.radT = (const T*)c->dt.radT;
   a.met = (const T*)c->dt.met;
   a.c2 = (const T*)c->dt.c2;
   a.runs = runs;
