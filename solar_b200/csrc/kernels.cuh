@@ -458,6 +458,7 @@ struct StageArgs {
   T dt, alpha, beta, inv_dxi;
   int kchunk;
   int tsel;                 // tiles launched: kTilesAll, kTilesInterior or kTilesRing
+  int store_w;              // MODE 0/5: write qw back (the last stage's register is never read)
 };
 
 // Tile subsets of a face (stage_tile).  The interior tiles (1..tx-2) x (1..ty-2) read no
@@ -777,7 +778,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
           w[q] = (MODE == 1) ? dt * r : fma(alpha, qwv[f][q], dt * r);
           o[q] = fma(beta, w[q], qv[q]);
         }
-        stv(qwS[f] + kp, w);
+        if (MODE == 1 || a.store_w) stv(qwS[f] + kp, w);
         stv(outS[f] + kp, o);
       };
       if (HAS_RHO) update(kRho, rho, r_rho, true);

@@ -495,6 +495,10 @@ static int launch_stage(solar_ctx* c, const void* qin, void* qout, int mode, int
   a.alpha = (T)kAlpha[stage];
   a.beta = (T)kBeta[stage];
   a.inv_dxi = (T)(1.0 / c->ht.dxi);
+  // Stage 1 of the next step starts from qw = 0 (alpha = 0), so the last stage does not write
+  // qw back: one of its four passes over the
+  // stored fields (6 x 128^3, us per step: 962 -> 922 in float, 2172 -> 2121 in double).
+  a.store_w = stage != 4;
   a.kchunk = c->kchunk;
   int tx = c->tile_x, ty = c->tile_y;
   if (mode == 2 || mode == 3) default_tile(c->g.n, c->fp32, &tx, &ty);   // operator-level calls
