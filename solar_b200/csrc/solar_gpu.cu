@@ -191,7 +191,8 @@ struct solar_ctx {
   double* norm_ring = nullptr; // per-step sums of squares (solar_gpu_rk4_norms)
   int norm_ring_len = 0;
   DevTables dt;
-  int tile_x = 32, tile_y = 8, kchunk = 0, edge_kchunk = 16;
+  int tile_x = 32, tile_y = 8, kchunk = 0;
+  int edge_resident = 0;       // edge-kernel CTAs per SM (threads and shared memory depend on nx)
   cudaGraphExec_t step_graph = nullptr;
   std::vector<cudaGraphExec_t> batch_graphs;   // batched step graph per number of live runs
   cudaEvent_t ev[8] = {};
@@ -354,7 +355,9 @@ static bool make_compact_map(const solar_ctx* c, const void* base, int bx, int b
 // positions [min s0t, max s0t + 9), widened to whole 16-byte pieces.
 static int edge_windows(solar_ctx* c) {
   const int n = c->g.n, w16 = c->fp32 ? 4 : 2;
-  const int ts = std::min(n, 128), nseg = (n + ts - 1) / ts;
+  // the fewest segments of at most 128 positions, all of the same length: with 128 + 32 at nx =
+  // 160 a quarter of the CTAs had 3/4 of their threads idle
+  const int nseg = (n + 127) / 128, ts = (n + nseg - 1) / nseg;
   std::vector<int> win((size_t)24 * nseg * 2);
   int sp = 0;
   for (int fe = 0; fe < 24; ++fe)
@@ -380,6 +383,24 @@ static int edge_windows(solar_ctx* c) {
   return SOLAR_OK;
 }
 
+// Planes per edge CTA for `lines` CTAs per chunk of the nk owned planes: waves x (planes + 3)
+// for the prologue's weights and the first loads, plus a term for the CTAs that share an SM.
+// us per step at 6 x 64^3, double: 6 planes in 0.9 waves 353, 4 in 1.3 waves 369 and the former
+// 8 planes (two CTAs per SM whatever their size) 370; 12 runs of 6 x 64^3, float: 22 planes in
+// 1.95 waves 1710, 64 in 0.65 waves 1774; 6 x 32^3, double: 3 planes 90.0, 2 and 4 planes
+// 89.9 and 92.2, 6 planes 98.4, 1 plane 96.8.
+static int edge_planes(long long lines, int nk, int nsm, int resident) {
+  int best = nk;
+  double best_cost = 0.0;
+  for (int nch = 1; nch <= nk; ++nch) {
+    const int kc = (nk + nch - 1) / nch;
+    const double units = (double)(lines * ((nk + kc - 1) / kc));
+    const double cost = std::ceil(units / ((double)nsm * resident)) * (kc + 3.0) + units / (1.1 * nsm);
+    if (nch == 1 || cost < best_cost) { best_cost = cost; best = kc; }
+  }
+  return best;
+}
+
 template <typename T>
 static int launch_edge(solar_ctx* c, void* buf, int mode, const int* runs) {
   EdgeArgs<T> a;
@@ -395,13 +416,7 @@ static int launch_edge(solar_ctx* c, void* buf, int mode, const int* runs) {
   a.nseg = c->dt.ewin_nseg;
   a.sp = c->dt.ewin_sp;
   a.ngroups = mode == 1 ? (c->g.nf + 1) / 2 : 2;
-  // About one wave of resident CTAs, each marching at least 4 planes.
   const int nrl = launched_runs(c, runs);
-  const long long per_chunk = 4LL * c->g.nface * a.ngroups * a.nseg * nrl;
-  const long long slots = (long long)c->nsm * EdgeMinBlocks<T>::value;
-  const long long nch = std::max<long long>(1, slots / per_chunk);
-  const int nk = c->g.k1 - c->g.k0;
-  a.kchunk = std::max<int>(4, (int)((nk + nch - 1) / nch));
   const size_t smem = (size_t)edge_smem_bytes(a.sp, a.ts, (int)sizeof(T));
   // a tile box side is at most 256 values; each thread spreads at most one row
   if (smem > 200 * 1024 || a.sp > 256 || 2 * a.sp > 3 * a.ts)
@@ -414,9 +429,44 @@ static int launch_edge(solar_ctx* c, void* buf, int mode, const int* runs) {
     CK(cudaFuncSetAttribute(edge_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attr_set = true;
   }
+  const int nk = c->g.k1 - c->g.k0;
+  const long long lines = 4LL * c->g.nface * a.ngroups * a.nseg * nrl;
+  if (!c->edge_resident) {
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->edge_resident, edge_kernel<T>, 3 * a.ts, smem));
+    c->edge_resident = std::max(c->edge_resident, 1);
+  }
+  a.kchunk = edge_planes(lines, nk, c->nsm, c->edge_resident);
   dim3 grid((nk + a.kchunk - 1) / a.kchunk, 4 * c->g.nface * a.ngroups * a.nseg, nrl);
   CK(launch_pdl(edge_kernel<T>, grid, dim3(3 * a.ts), smem, c->stream, a));
   return SOLAR_OK;
+}
+
+// Radial planes per stage CTA when the descriptor names none: tiles of a face x volumes (faces
+// of every run) CTAs per chunk of the nk owned planes, `slots` resident CTAs on the device.
+//   float: waves x (planes + 2.5).  A CTA's prologue and ring fill cost about 2.5 planes, and up
+//     to a few waves the planes of a CTA take the same time whatever the other slots hold (6 x
+//     128^3, 64 x 8 tiles, us per step: 43 planes in 1.95 waves 958, 22 in 3.9 995, 32 in 2.6
+//     1042, 64 in 1.3 1263; 6 x 64^3: 11 planes in 0.97 waves 191, 16 in 1.3 230, 32 309).
+//   double is closer to the memory bound, so the fill hides behind the other CTA of the SM and
+//     long chunks lose the halo planes that neighbouring CTAs share in L2, 0.6% per plane (6 x
+//     128^3, 32 x 8 tiles: 11 planes in 15.6 waves 2162, 22 in 7.8 2252, 43 in 3.9 2389; 6 x
+//     32^3: 3 planes in 0.9 waves 100, 8 in 0.3 127, 2 in 1.3 119).
+//     A wave of few tiles per face spans many volumes, each its own stream of DRAM pages, the
+//     longer the chunks the more: 12 runs of 6 x 64^3 (8 tiles) take 16 planes 1775, 32 1782,
+//     64 1822, though 64 make the fewest CTAs.
+// The last of many waves overlaps the one before it, so past four waves the fraction counts too.
+static int plan_planes(int tiles, int volumes, int nk, long long slots, bool fp32) {
+  const long long columns = (long long)tiles * volumes;
+  int best = nk;
+  double best_cost = 0.0;
+  for (int nch = 1; nch <= nk; ++nch) {
+    const int kc = (nk + nch - 1) / nch;
+    const double w = (double)(columns * ((nk + kc - 1) / kc)) / (double)slots;
+    const double up = std::ceil(w), waves = w < 4.0 ? up : 0.6 * w + 0.4 * up;
+    const double cost = fp32 ? waves * (kc + 2.5) * (1.0 + 0.03 * kc / tiles) : waves * (kc + 0.5) * (1.0 + 0.006 * kc);
+    if (nch == 1 || cost < best_cost) { best_cost = cost; best = kc; }
+  }
+  return best;
 }
 
 template <typename T, int TX, int TY, int MODE, bool HAS_RHO, bool FORCE = false>
@@ -434,10 +484,21 @@ static int launch_stage_t(solar_ctx* c, StageArgs<T>& a, const void* qin) {
   }
   const size_t smem = a.c2 ? L::TOTAL_C2 : L::TOTAL;
   if (!a.c2) a.mC2 = a.mO;                         // unused
-  const int nchunks = (c->g.k1 - c->g.k0 + a.kchunk - 1) / a.kchunk;
   const int ntiles = stage_tile_count(a.tsel, c->g.n / TX, c->g.n / TY);
   if (ntiles <= 0) return SOLAR_OK;                // no interior tiles at this size
-  dim3 grid(ntiles, nchunks, launched_runs(c, a.runs) * c->g.nface);
+  const int nk = c->g.k1 - c->g.k0, volumes = launched_runs(c, a.runs) * c->g.nface;
+  if (a.kchunk <= 0) {
+    static int resident[2] = {0, 0};               // CTAs per SM without / with the c^2 boxes
+    int& res = resident[a.c2 ? 1 : 0];
+    if (!res) {
+      int r = 1;
+      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, stage_kernel<T, TX, TY, MODE, HAS_RHO, FORCE>,
+                                                       TX / Vec16<T>::V * TY, smem));
+      res = std::max(r, 1);
+    }
+    a.kchunk = plan_planes(ntiles, volumes, nk, (long long)c->nsm * res, c->fp32);
+  }
+  dim3 grid(ntiles, (nk + a.kchunk - 1) / a.kchunk, volumes);
   CK(launch_pdl(stage_kernel<T, TX, TY, MODE, HAS_RHO, FORCE>, grid, dim3(TX / Vec16<T>::V, TY), smem, c->stream, a));
   return SOLAR_OK;
 }
@@ -465,14 +526,15 @@ static int launch_stage_mode(solar_ctx* c, StageArgs<T>& a, const void* qin, int
   }
 }
 
-// Stage tiles (TX x TY points).  The default is 64 x 8 when nx is a multiple of 64 (the
-// fastest shape measured at 64^3, 128^3 and 384^3 in both precisions), else 32 x 16 in
-// float and 32 x 8 in double, and 16 x 16 when nx is not a multiple of 32.
+// Stage tiles (TX x TY points) when the descriptor names none.  Float: 64 x 8 when nx is a
+// multiple of 64, else 32 x 8 (us per step with the best radial chunks, 64 x 8 / 32 x 8 / 32 x
+// 16: 6 x 192^2 x 120 1904 / 1926 / 1943, 6 x 128^3 958 / 972 / 976; 6 x 96^3 - / 492 / 494, 6 x
+// 32^3 - / 76 / 78).  Double: 32 x 8 (6 x 128^3 2162 for 32 x 8, 2209 for 64 x 8; 6 x 64^3 382,
+// 383; 6 x 160^2 x 96 2537 for 32 x 8, 2601 for 32 x 16).  16 x 16 when nx is not a multiple of 32.
 static void default_tile(int n, bool fp32, int* tx, int* ty) {
   if (n % 32) { *tx = 16; *ty = 16; return; }
-  if (n % 64 == 0) { *tx = 64; *ty = 8; return; }
-  *tx = 32;
-  *ty = fp32 ? 16 : 8;
+  *tx = fp32 && n % 64 == 0 ? 64 : 32;
+  *ty = 8;
 }
 
 template <typename T>
@@ -546,6 +608,13 @@ static int launch_filter_t(solar_ctx* c, const void* qin, void* qout, const int*
   if (units > slots) {
     cut = units % slots;
     if (cut > 0) chunks = std::min<long long>(nk / 11, std::max<long long>(1, (slots + cut / 2) / cut));
+  } else if (2 * units <= slots && nk >= 22) {
+    // Two or more chunks of every unit fit in one wave: the march through the planes is the
+    // kernel's time, so every unit is cut (us per step at 6 x 64^3, float: 3 chunks 175, whole
+    // columns and 44 cut ones 185; 6 x 32^3: 2 chunks 69.7 in float, 93.5 in double, whole 73.8,
+    // 98.4; chunks shorter than 11 planes gain nothing, they re-read 10).
+    cut = units;
+    chunks = std::min<long long>(nk / 11, slots / units);
   } else {
     const long long per = units / c->nsm;
     cut = units % c->nsm;
@@ -945,22 +1014,7 @@ int solar_gpu_init(const solar_desc* d, solar_ctx** out) {
       return fail(SOLAR_ERR_ARG, "unsupported stage tile %d x %d for nx %d", tx, ty, nx);
     }
   }
-  if (d->kchunk > 0) c->kchunk = d->kchunk;
-  else {
-    // Radial planes per stage CTA.  Measured best on B200: about nr/3 in float and nr/6 in
-    // double, between 16 and 64 (43 / 22 at 128^3, 64 at 384^3, ~21 at 64 runs of 64^3).
-    // Grids too small to fill one wave of two CTAs per SM that way get about four waves.
-    const long long blocks = 6LL * g.nruns * (g.n / c->tile_x) * (g.n / c->tile_y);
-    int kc = std::min(64, std::max(16, c->fp32 ? g.nr / 3 : g.nr / 6));
-    int nch = (g.nr + kc - 1) / kc;
-    if (blocks * nch < 148LL * 2) {
-      const long long want = 148LL * 2 * 4;
-      nch = (int)std::max<long long>(1, (want + blocks - 1) / blocks);
-      c->kchunk = std::max(8, (g.nr + nch - 1) / nch);
-    } else {
-      c->kchunk = (g.nr + nch - 1) / nch;
-    }
-  }
+  c->kchunk = std::max(0, d->kchunk);   // 0: chosen per launch (plan_planes)
 #define TRY(x) do { int rc_ = (x); if (rc_) { solar_gpu_finalize(c); return rc_; } } while (0)
 #define TRYC(call) do { cudaError_t e_ = (call); if (e_ != cudaSuccess) { std::string m_ = cudaGetErrorString(e_); solar_gpu_finalize(c); return fail(e_ == cudaErrorMemoryAllocation ? SOLAR_ERR_NOMEM : SOLAR_ERR_CUDA, "%s: %s", #call, m_.c_str()); } } while (0)
   TRYC(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));

@@ -58,3 +58,37 @@ def test_rhs_with_3d_sound_speed_and_source(oracle_mod, cfg, state, c2):
         got, want = s.compute_rhs(state), o.compute_rhs(state)
     for m in range(5):
         assert rel_l2(got[:, m], want[:, m]) <= 1e-12, m
+
+
+@pytest.mark.parametrize("nx,nr", [(16, 16), (32, 22), (48, 47), (144, 17), (272, 16)])
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-11), ("fp32", 1e-5)])
+def test_default_shapes(oracle_mod, nx, nr, precision, tol):
+    """Shapes the library chooses itself: one step, which passes every kernel, where the radial
+    chunks of the edge and filter kernels leave remainders (48 x 47), where the filter cuts
+    every column in two (32 x 22, the smallest that is cut) and where an edge takes two and
+    three segments (144: 72 positions each; 272: 91, 91 and 90)."""
+    cfg = configs.c2(nx=nx, nr=nr)
+    q = np.random.default_rng(nx).standard_normal((6, 5, nr, nx, nx))
+    want = oracle_mod.Oracle(cfg).rk4(q, 1)
+    with Solver(cfg, precision=precision, tuned=False) as s:
+        s.set_state(q)
+        s.rk4(1)
+        got = s.get_state()
+    for m in range(5):
+        assert rel_l2(got[:, m], want[:, m]) <= tol, m
+
+
+def test_batch_shapes_follow_the_live_runs(oracle_mod):
+    """The launch shapes of a batch depend on how many runs are live; every run still equals the oracle's."""
+    cfg = configs.c2(nx=32, nr=27)
+    steps = [1, 3, 2, 3, 0]
+    q = np.random.default_rng(3).standard_normal((len(steps), 6, 5, 27, 32, 32))
+    o = oracle_mod.Oracle(cfg)
+    with Solver(cfg, nruns=len(steps)) as s:
+        for r in range(len(steps)):
+            s.set_state(q[r], r)
+        s.rk4_runs(steps)
+        for r, n in enumerate(steps):
+            got, want = s.get_state(r), o.rk4(q[r], n)
+            for m in range(5):
+                assert rel_l2(got[:, m], want[:, m]) <= 1e-11, (r, m)
