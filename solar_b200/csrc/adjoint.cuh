@@ -8,13 +8,12 @@
 // and the gradient of a misfit with respect to a per-point sound-speed perturbation dc
 // (c -> c + dc enters only r_p = -c^2 rho0 div v, compute_rhs_acoustic.f90:134) gathers
 //     g += dt (-2 c rho0 div(v_{s-1})) mu_s^p            (0 on the BC planes).
-// L^T is applied in three kernels:
-//   adj_stage  mu, the BC mask, the pointwise terms, the sponge, lw and g, and the
-//              transposed derivatives of the coefficient-weighted fields: -D_xi and -D_eta
-//              with zero halos (the DRP stencil is antisymmetric) and the banded radial
-//              transpose, on the interior and on the ghost frame -- the frame values are the
-//              adjoints of the neighbour faces' ghost values;
-//   adj_rbdy   the one-sided (Tam-Dong) rows of the radial transpose;
+// L^T is applied in two kernels:
+//   adj_stage  mu, the BC mask, the pointwise terms, the sponge, g, and the transposed
+//              derivatives of the coefficient-weighted fields: -D_xi and -D_eta with zero
+//              halos (the DRP stencil is antisymmetric) and the radial transpose with its
+//              one-sided (Tam-Dong) rows, on the interior and on the ghost frame -- the frame
+//              values are the adjoints of the neighbour faces' ghost values;
 //   adj_edge   the transpose of the edge exchange: each source-line point gathers the ghost
 //              adjoints that used it, with the same folded coefficients.
 // FILTER_EXP^T is the radial transpose, then eta, then xi, each with its ghost-frame
@@ -25,74 +24,97 @@
 
 namespace solar {
 
-// Fused transposed stage (pointwise part + transposed stencils in one pass).  A CTA owns a
-// TX x TY column tile of one face and marches the planes of its chunk (plus three planes on
-// either side for the radial window).  Planes stream in through TMA tile loads into a ring of
-// shared-memory slots, each guarded by an mbarrier: for a plane of the chunk, the lambda_q
-// and lambda_w boxes (tile plus a 4-column / 3-row halo) of v_xi, v_eta, p and rho and the
-// tiles of v_r; for the three extra planes on either side only the tiles of p, rho and v_r.
-// Every plane also brings its c^2 box (the halo points use it too), the stored divergence
-// tile (chunk planes) and its row of radial coefficients (an untiled bulk copy), so the
-// per-plane values need no global loads.  Per plane the kernel forms the coefficient-weighted volumes X1, X2 (on the tile and its
-// xi halo) and Y1, Y2 (tile and eta halo) in shared memory from mu = lw + beta lq (zero
-// outside the face and on the BC planes), applies -D_xi / -D_eta, and keeps facr * R1 and
-// facr * R2 of the last seven planes in registers for the banded part of the radial
-// transpose, which completes plane k three iterations later.  The rows of the one-sided
-// radial stencil (planes 1, 2, nr-3, nr-2; planes 0 and nr-1 carry zero) are written to
-// `rb` and added by adj_rbdy_kernel.  Edge tiles also write the ghost-frame adjoints.
-// Inputs (lq, lw) and outputs (lout, lwout) are distinct buffers: neighbouring CTAs read the
-// inputs' halos.
+// Fused transposed stage (pointwise part + transposed stencils in one pass).  The register
+// lambda_w of the recursion above is never stored: with mu_s = lw_s + beta_s lq_s the
+// recursion is
+//     lq_{s-1} = lq_s + dt L^T(mu_s) ,   mu_{s-1} = alpha_s mu_s + beta_{s-1} lq_{s-1} ,
+// so the buffers hold lambda_q and mu, and only mu (whose neighbours the stencils read) comes
+// with a halo.  The step's first transposed stage (s = 5, where lw = 0) forms mu = beta lq from
+// lambda_q alone; its last (s = 1) writes no mu.
+//
+// A CTA owns a TX x TY column tile of one face and marches the planes of its chunk (plus three
+// planes on either side for the radial window).  Each thread owns V consecutive points of a row
+// (V = 16 bytes / sizeof(T)).  Planes stream in through TMA tile loads into a ring of
+// shared-memory slots, each guarded by an mbarrier: for a plane of the chunk the boxes of mu
+// (tile plus a 4-column / 3-row halo) of v_xi, v_eta, p and rho, the tile of v_r, the lambda_q
+// tiles, the c^2 box, the stored divergence, the gradient accumulator and the row of radial
+// coefficients; for the three
+// extra planes on either side the tiles of p, v_r, rho and c^2.  Per plane the kernel forms the
+// coefficient-weighted volumes X1, X2 (on the tile and its xi halo) and Y1, Y2 (tile and eta
+// halo) in shared memory (zero outside the face and on the BC planes; every thread takes its
+// own vector and at most one halo vector), and after one barrier applies -D_xi / -D_eta.  The
+// exchange arrays are double-buffered and a slot is read before the barrier only, so that one
+// barrier per plane serves both and thread 0 refills the slot right after it.  The banded
+// radial transpose adds each plane's facr * R1, facr * R2 to the partial outputs of the planes
+// m-3 .. m+3, held in registers; a plane is complete three iterations later.  The one-sided
+// rows of the radial stencil (planes 1, 2, nr-3, nr-2; planes 0 and nr-1 carry zero) reach the
+// seven planes at each end: a chunk that holds some of them reads those rows' points itself.
+// Edge tiles also write the ghost-frame adjoints.  Inputs (lambda_q, mu) and outputs are
+// distinct buffers: neighbouring CTAs read the inputs' halos.
 template <typename T>
 struct AdjStageArgs {
-  CUtensorMap mBq, mBw;   // boxes (TX+8) x (TY+6) of lq / lw
-  CUtensorMap mTq, mTw;   // tiles TX x TY of lq / lw
-  CUtensorMap mC2;        // boxes (TX+8) x (TY+6) of the compact c^2 (when present; zero outside the face)
+  CUtensorMap mB3;        // boxes (TX+8) x (TY+6) of mu (of lambda_q in the first stage): (rho,) v_xi, v_eta
+  CUtensorMap mB;         // box of p
+  CUtensorMap mM;         // tiles TX x TY of the same buffer: v_r; v_r, p
+  CUtensorMap mM2;
+  CUtensorMap mQ;         // tiles TX x TY of all fields of lambda_q (not in the first stage)
+  CUtensorMap mC2, mC2t;  // boxes and tiles of the compact c^2 (when present; zero outside the face)
   CUtensorMap mDiv;       // tiles TX x TY of the compact stored divergence (when present)
+  CUtensorMap mGrad;      // tiles TX x TY of the gradient accumulator (double, when present)
+  const T* mu;            // the buffer of mB
   T* lout;
-  T* lwout;
-  T* rb;              // [face][4][2][n*n] raw R1, R2 of planes 1, 2, nr-3, nr-2
-  const T* div;       // compact stage-input divergence, or nullptr
+  T* muout;               // nullptr in the last stage
+  const T* div;           // compact stage-input divergence, or nullptr
   const T* c2;
-  double* grad;
-  const T* rad;
+  double* grad;           // sum over the stages of dt rho0 div mu_p (grad_scale_kernel: -2 c)
   const T* met;
-  const T* radT;      // [nr][16]: the radial rows of a plane together (through the ring)
-  WaitCtl wc;         // error word and bound of the ring waits
+  const T* radT;          // [nr][16]: the radial rows of a plane together (through the ring)
+  WaitCtl wc;             // error word and bound of the ring waits
   Geom g;
-  T alpha, beta, dt, inv_dxi;
-  int keep, kchunk;
+  T alpha, beta, beta_next, dt, inv_dxi;   // mu = beta * box (1 but in the first stage)
+  int first, keep, kchunk;
 };
 
-// Ring slots: two in both precisions.  In float that leaves room for three CTAs per SM
-// (80 registers, 54 KB of shared memory each): reverse sweep at 6 x 96^3 4.4% faster than
-// three slots with two CTAs; four CTAs (64 registers, a 16-byte spill) gained less (1.1%).
-template <typename T> struct AdjRing { static constexpr int value = 2; };
+// What bounds it: the latency of a plane's loads.  Requests count as much as bytes: with one TMA
+// request per field (14 per plane in double) a reverse step at 6 x 96^3 took 2045 us in double and
+// 850 in float, with the fields of one shape in one 4-D request (8 per plane) 1681 and 838.  Two
+// slots keep two CTAs per SM in double (110 KB each) and four in float (51 KB).  The form before
+// (one point per thread, lambda_w and lambda_q boxes, two barriers per plane, a kernel of its own
+// for the one-sided rows) took 2163 and 1198.
+constexpr int kAdjRing = 2;
 
-template <typename T, int TX, int TY>
+template <typename T, int TX, int TY, bool HAS_RHO>
 struct AdjLayout {
-  static constexpr int PW = TX + 8, PH = TY + 6, PB = PW * PH, OB = TX * TY;
+  static constexpr int V = Vec16<T>::V, NTH = TX / V * TY;
+  static constexpr int PW = TX + 8, YH = TY + 6, PB = PW * YH, OB = TX * TY;
+  static constexpr int NB = HAS_RHO ? 4 : 3, NF = NB + 1;
   static constexpr size_t P_BYTES = align128(PB * sizeof(T));
   static constexpr size_t O_BYTES = align128(OB * sizeof(T));
-  // a chunk plane: boxes [v_xi, v_eta, p, rho] x [lq, lw], then the v_r tiles [lq, lw];
-  // an extra plane: tiles [p, rho, v_r] x [lq, lw] from the slot's start; every plane: the
-  // c^2 box (the halo points read it too) and (chunk planes) the stored-divergence tile
-  // after it, then the plane's row of radial coefficients (16 values, zero padded)
-  static constexpr size_t AUX = 8 * P_BYTES + 2 * O_BYTES;
-  static constexpr size_t DIV_OFF = AUX + P_BYTES;
-  static constexpr size_t RAD_OFF = DIV_OFF + O_BYTES;
-  static constexpr size_t SLOT = align128(RAD_OFF + 16 * sizeof(T));
-  static constexpr int RING = AdjRing<T>::value;
-  static constexpr size_t BAR = RING * SLOT;
-  static constexpr size_t TOTAL = BAR + RING * sizeof(uint64_t);
+  // a chunk plane: boxes of mu [(rho,) v_xi, v_eta] as one load, [p], the tile of v_r, the
+  // lambda_q tiles of every field in storage order as one load; an extra plane: tiles [v_r, p]
+  // as one load, [rho], from the slot's start
+  static constexpr size_t PBOX = align128((NB - 1) * PB * sizeof(T)), VR = PBOX + P_BYTES;
+  static constexpr size_t LQ = VR + O_BYTES, C2 = LQ + NF * O_BYTES;
+  static_assert(OB * sizeof(T) % 128 == 0, "tiles of one load follow each other");
+  static constexpr size_t DIV = C2 + P_BYTES, GRAD = DIV + O_BYTES, RAD = GRAD + align128(OB * sizeof(double));
+  static constexpr size_t SLOT = align128(RAD + 16 * sizeof(T));
+  static constexpr int XB = TY * PW, YB = YH * TX;                  // exchange arrays
+  static constexpr size_t EX = kAdjRing * SLOT;                     // [2][X1, X2, Y1, Y2]
+  static constexpr size_t EX_BYTES = 2 * (XB + YB) * sizeof(T);
+  static constexpr size_t ONE = EX + 2 * EX_BYTES;                  // one-sided rows, [4][NTH] vectors
+  static constexpr size_t BAR = ONE + (size_t)4 * NTH * 16;
+  static constexpr size_t TOTAL = BAR + kAdjRing * sizeof(uint64_t);
 };
 
-template <typename T, int TX, int TY>
-__global__ void __launch_bounds__(TX * TY, sizeof(T) == 4 ? 3 : 2) adj_stage_kernel(const __grid_constant__ AdjStageArgs<T> a) {
-  using L = AdjLayout<T, TX, TY>;
-  constexpr int XW = TX + 6, YH = TY + 6, PW = L::PW;
-  constexpr int NHALO = 6 * TX + 6 * TY;
-  static_assert(NHALO <= TX * TY, "one halo point per thread");
-  __shared__ T sX1[TY][XW], sX2[TY][XW], sY1[YH][TX], sY2[YH][TX];
+template <typename T, int TX, int TY, bool HAS_RHO>
+__global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const __grid_constant__ AdjStageArgs<T> a) {
+  using L = AdjLayout<T, TX, TY, HAS_RHO>;
+  constexpr int V = L::V, NT = TX / V, PW = L::PW, YH = L::YH;
+  constexpr int QV = 4 / V;                          // vectors in the 4-column margin of a box
+  constexpr int NETA = 6 * NT, NXI = 2 * QV * TY;    // halo vectors
+  constexpr int NV = (V + 8) / V;                    // vectors covering columns c-4 .. c+V+3
+  constexpr int PBs = L::PB, OBs = L::OB, R0 = HAS_RHO ? 1 : 0;   // storage slots: (rho,) v_xi, v_eta, v_r, p
+  static_assert(NETA + NXI <= L::NTH, "one halo vector per thread");
   extern __shared__ __align__(128) unsigned char smem[];
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
   const Geom& g = a.g;
@@ -103,300 +125,407 @@ __global__ void __launch_bounds__(TX * TY, sizeof(T) == 4 ? 3 : 2) adj_stage_ker
   const int face = blockIdx.z;
   const int kb = blockIdx.y * a.kchunk, ke = min(nr, kb + a.kchunk);
   if (kb >= nr) return;
-  const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
-  const int i = i0 + tx, j = j0 + ty;
-  const int p2 = j * n + i;
+  const int cx = threadIdx.x, ty = threadIdx.y, tid = ty * NT + cx;
   const int sRho = g.slot[kRho], sX = g.slot[kVxi], sY = g.slot[kVeta], sR = g.slot[kVr], sP = g.slot[kP];
-  const bool has_rho = sRho >= 0;
-  const T* __restrict__ met = a.met;
   const T c1 = Coef<T>::drp(1), c2c = Coef<T>::drp(2), c3 = Coef<T>::drp(3);
-  // this thread's halo point: eta-halo rows first, then xi-halo columns
-  const bool has_halo = tid < NHALO;
-  bool xi_halo = false;
-  int hi = 0, hj = 0;
-  if (tid < 6 * TX) { hi = tid % TX; const int r = tid / TX; hj = r < 3 ? r - 3 : TY + r - 3; }
-  else if (has_halo) { xi_halo = true; const int q = tid - 6 * TX; hj = q % TY; const int cc = q / TY; hi = cc < 3 ? cc - 3 : TX + cc - 3; }
-  const int hgi = i0 + hi, hgj = j0 + hj;
-  const bool h_in = has_halo && hgi >= 0 && hgi < n && hgj >= 0 && hgj < n;
-  const int hq2 = h_in ? hgj * n + hgi : 0;
-  // 32-bit offsets inside one field volume; the field bases of this face are formed once
-  T* const lo_face = a.lout + g.vol(0, face, 0);
-  T* const lw_face = a.lwout + g.vol(0, face, 0);
-  const int vs = (int)g.vs, plane = (int)g.plane;
-  auto fo = [&](int s) { return s * vs; };                          // field base (elements)
-  const int own0 = (JOFF + j) * g.pitch + IOFF + i;                 // own point in plane 0
-  const int face_c2 = face * nr;                                    // plane index base, compact arrays
-  // planes loaded through the ring: every real plane of [kb-3, ke+2]
-  const int m_lo = max(kb - 3, 0), m_hi = min(ke + 2, nr - 1);
-  const int zf = face * g.nf;            // plane index of (slot s, k) = (zf + s) * nr + k (run 0)
-  const int xB = IOFF + i0 - 4, yB = JOFF + j0 - 3, xT = IOFF + i0, yT = JOFF + j0;
-  auto slot_base = [&](int sl) { return smem + (size_t)sl * L::SLOT; };
-  const bool tc2 = a.c2 != nullptr, tdiv = a.grad != nullptr;   // c^2 / divergence tiles in the ring
-  const int zc = face * nr;                // plane index of the compact arrays: face * nr + k
-  auto issue = [&](int m, int sl) {
-    uint64_t* bar = &bars[sl];
-    unsigned char* base = slot_base(sl);
-    const bool chunk = m >= kb && m < ke;
-    if (tc2) tma_load_3d(base + L::AUX, &a.mC2, i0 - 4, j0 - 3, zc + m, bar);
-    if (tdiv && chunk) tma_load_3d(base + L::DIV_OFF, &a.mDiv, i0, j0, zc + m, bar);
-    bulk_load(base + L::RAD_OFF, a.radT + (size_t)m * 16, 16 * sizeof(T), bar);
-    const uint32_t aux = (uint32_t)(((tc2 ? L::PB : 0) + (tdiv && chunk ? L::OB : 0) + 16) * sizeof(T));
-    if (chunk) {
-      const int nbox = has_rho ? 4 : 3;
-      mbar_expect_tx(bar, (uint32_t)((2 * nbox * L::PB + 2 * L::OB) * sizeof(T)) + aux);
-      const int bs[4] = {sX, sY, sP, sRho};
-      for (int f = 0; f < nbox; ++f) {
-        tma_load_3d(base + (2 * f) * L::P_BYTES, &a.mBq, xB, yB, (zf + bs[f]) * nr + m, bar);
-        tma_load_3d(base + (2 * f + 1) * L::P_BYTES, &a.mBw, xB, yB, (zf + bs[f]) * nr + m, bar);
-      }
-      tma_load_3d(base + 8 * L::P_BYTES, &a.mTq, xT, yT, (zf + sR) * nr + m, bar);
-      tma_load_3d(base + 8 * L::P_BYTES + L::O_BYTES, &a.mTw, xT, yT, (zf + sR) * nr + m, bar);
-    } else {
-      const int nt = has_rho ? 3 : 2;
-      mbar_expect_tx(bar, (uint32_t)(2 * nt * L::OB * sizeof(T)) + aux);
-      const int ts[3] = {sP, sR, sRho};
-      for (int f = 0; f < nt; ++f) {
-        tma_load_3d(base + (2 * f) * L::O_BYTES, &a.mTq, xT, yT, (zf + ts[f]) * nr + m, bar);
-        tma_load_3d(base + (2 * f + 1) * L::O_BYTES, &a.mTw, xT, yT, (zf + ts[f]) * nr + m, bar);
-      }
-    }
-  };
+  const int p2 = (j0 + ty) * n + i0 + V * cx;        // first own point
+  // this thread's halo vector: the eta-halo rows first, then the xi-halo columns
+  const bool has_halo = tid < NETA + NXI, xi_halo = tid >= NETA;
+  int hi, hj;
+  if (!xi_halo) {
+    const int r = tid / NT;
+    hi = (tid % NT) * V;
+    hj = r < 3 ? r - 3 : TY + r - 3;
+  } else {
+    const int q = (tid - NETA) / TY;
+    hi = q < QV ? q * V - 4 : TX + (q - QV) * V;
+    hj = (tid - NETA) % TY;
+  }
+  const bool h_in = has_halo && i0 + hi >= 0 && i0 + hi < n && j0 + hj >= 0 && j0 + hj < n;
+  const int hq2 = h_in ? (j0 + hj) * n + i0 + hi : 0;
+  const int hb = (hj + 3) * PW + hi + 4;             // in a box
+  // The 2-D metric terms of the own and of the halo points sit in registers for the chunk.
+  T gD[V], gXYD[V], gC[V], gXYC[V], gDivX[V], gDivY[V], gTX[V], gTY[V], gh1[V], gh2[V], gh3[V];
+  ldv(a.met + mD * P2 + p2, gD);
+  ldv(a.met + mXYD * P2 + p2, gXYD);
+  ldv(a.met + mC * P2 + p2, gC);
+  ldv(a.met + mXYC * P2 + p2, gXYC);
+  ldv(a.met + mDivX * P2 + p2, gDivX);
+  ldv(a.met + mDivY * P2 + p2, gDivY);
+  ldv(a.met + mTX * P2 + p2, gTX);
+  ldv(a.met + mTY * P2 + p2, gTY);
+  ldv(a.met + (xi_halo ? mD : mXYD) * P2 + hq2, gh1);
+  ldv(a.met + (xi_halo ? mXYC : mC) * P2 + hq2, gh2);
+  ldv(a.met + (xi_halo ? mDivX : mDivY) * P2 + hq2, gh3);
   if (tid == 0) {
-    for (int q = 0; q < L::RING; ++q) mbar_init(&bars[q], 1);
+    for (int q = 0; q < kAdjRing; ++q) mbar_init(&bars[q], 1);
     mbar_fence_init();
   }
   __syncthreads();
-  // planes [m_lo, m_issued) have loads issued; thread 0 has seen planes [m_lo, m_seen) land
+  // programmatic launch: everything above reads constant tables only
+  grid_dependency_wait();
+
+  // 32-bit offsets inside one face's volumes
+  T* const lo_face = a.lout + g.vol(0, face, 0);
+  T* const mu_face = a.muout ? a.muout + g.vol(0, face, 0) : nullptr;
+  const int vs = (int)g.vs, plane = (int)g.plane;
+  const int own0 = (int)g.at(0, j0 + ty, i0 + V * cx);              // own points in plane 0
+  const int zf = face * g.nf;            // plane index of (slot s, k) = (zf + s) * nr + k (run 0)
+  const int xB = IOFF + i0 - 4, yB = JOFF + j0 - 3, xT = IOFF + i0, yT = JOFF + j0;
+  const bool tc2 = a.c2 != nullptr, tdiv = a.grad != nullptr;
+  auto slot_base = [&](int sl) { return smem + (size_t)sl * L::SLOT; };
+  auto issue = [&](int m, int sl) {
+    uint64_t* bar = &bars[sl];
+    unsigned char* base = slot_base(sl);
+    const int zc = face * nr + m;        // plane index of the compact arrays
+    const bool chunk = m >= kb && m < ke;
+    uint32_t values = 16;
+    if (chunk) values += L::NB * L::PB + L::OB + (a.first ? 0 : L::NF * L::OB) + (tc2 ? L::PB : 0) + (tdiv ? L::OB + L::OB * (sizeof(double) / sizeof(T)) : 0);
+    else values += (L::NB - 1 + (tc2 ? 1 : 0)) * L::OB;
+    mbar_expect_tx(bar, values * (uint32_t)sizeof(T));
+    bulk_load(base + L::RAD, a.radT + (size_t)m * 16, 16 * sizeof(T), bar);
+    if (chunk) {
+      tma_load_4d(base, &a.mB3, xB, yB, m, zf, bar);
+      tma_load_3d(base + L::PBOX, &a.mB, xB, yB, (zf + sP) * nr + m, bar);
+      tma_load_3d(base + L::VR, &a.mM, xT, yT, (zf + sR) * nr + m, bar);
+      if (!a.first) tma_load_4d(base + L::LQ, &a.mQ, xT, yT, m, zf, bar);
+      if (tc2) tma_load_3d(base + L::C2, &a.mC2, i0 - 4, j0 - 3, zc, bar);
+      if (tdiv) {
+        tma_load_3d(base + L::DIV, &a.mDiv, i0, j0, zc, bar);
+        tma_load_3d(base + L::GRAD, &a.mGrad, i0, j0, zc, bar);
+      }
+    } else {
+      tma_load_4d(base, &a.mM2, xT, yT, m, zf + sR, bar);
+      if (HAS_RHO) tma_load_3d(base + 2 * L::O_BYTES, &a.mM, xT, yT, (zf + sRho) * nr + m, bar);
+      if (tc2) tma_load_3d(base + L::C2, &a.mC2t, i0, j0, zc, bar);
+    }
+  };
+  // planes loaded through the ring: every real plane of [kb-3, ke+2]; planes [m_lo, m_issued)
+  // have loads issued, thread 0 has seen planes [m_lo, m_seen) land
+  const int m_lo = max(kb - 3, 0), m_hi = min(ke + 2, nr - 1);
   int m_issued = m_lo, m_seen = m_lo;
   const bool loads = !a.wc.no_loads;
   if (tid == 0 && loads) {
-    tma_prefetch_desc(&a.mBq);
-    tma_prefetch_desc(&a.mBw);
-    for (int q = 0; q < L::RING && m_issued <= m_hi; ++q, ++m_issued) issue(m_issued, q);
+    tma_prefetch_desc(&a.mB);
+    for (int q = 0; q < kAdjRing && m_issued <= m_hi; ++q, ++m_issued) issue(m_issued, q);
   }
-  T w1[7], w2[7];          // facr * R1, facr * R2 of planes m-6 .. m (banded rows only)
-  T pp[4], pv[4];          // partial outputs of p and v_r, planes m-3 .. m
+  // facr * dt * (R1, R2) of one of the one-sided rows, from global memory
+  auto one_sided = [&](int kk, int row) {
+    const T* rr = a.radT + (size_t)kk * 16;
+    const T* src = a.mu + g.vol(0, face, 0) + (long long)kk * plane + own0;
+    T vp[V], vv[V], vrho[V], cc[V], r1[V], r2[V];
+    ldv(src + (long long)sP * vs, vp);
+    ldv(src + (long long)sR * vs, vv);
+    if (HAS_RHO) ldv(src + (long long)sRho * vs, vrho);
+    if (tc2) ldv(a.c2 + ((long long)face * nr + kk) * P2 + p2, cc);
+    const T f = a.dt * rr[rFacR], rho0 = rr[rRho0];
 #pragma unroll
-  for (int q = 0; q < 7; ++q) { w1[q] = T(0); w2[q] = T(0); }
+    for (int q = 0; q < V; ++q) {
+      const T c2rho0 = tc2 ? cc[q] * rho0 : rr[rC2Rho0];
+      r1[q] = -f * rr[rInvRho0] * (a.beta * vv[q]);
+      r2[q] = -f * (c2rho0 * (a.beta * vp[q]) + (HAS_RHO ? rho0 * (a.beta * vrho[q]) : T(0)));
+    }
+    T* d = reinterpret_cast<T*>(smem + L::ONE) + (size_t)tid * V;
+    stv(d + (2 * row) * L::NTH * V, r1);
+    stv(d + (2 * row + 1) * L::NTH * V, r2);
+  };
+  if (kb <= 6) { one_sided(1, 0); one_sided(2, 1); }
+
+  T ap[7][V], av[7][V];          // partial outputs of p and v_r, planes m-3 .. m+3
+  T kp[4][V], kv[4][V];          // alpha * mu of p and v_r, planes m-3 .. m
 #pragma unroll
-  for (int q = 0; q < 4; ++q) { pp[q] = T(0); pv[q] = T(0); }
-  // The 2-D metric terms of the own point and of the halo point are the same on every plane
-  // and are held in registers for the whole chunk (the per-plane reads were the kernel's
-  // main long-scoreboard stall).  In double this spills 28 bytes under the 128-register
-  // budget and still ran 1% faster than four 16-byte reads per plane.
-  const T gD = __ldg(met + mD * P2 + p2), gXYD = __ldg(met + mXYD * P2 + p2);
-  const T gC = __ldg(met + mC * P2 + p2), gXYC = __ldg(met + mXYC * P2 + p2);
-  const T gDivX = __ldg(met + mDivX * P2 + p2), gDivY = __ldg(met + mDivY * P2 + p2);
-  const T gTX = __ldg(met + mTX * P2 + p2), gTY = __ldg(met + mTY * P2 + p2);
-  T gh1 = T(0), gh2 = T(0), gh3 = T(0);
-  if (h_in) {
-    gh1 = __ldg(met + (xi_halo ? mD : mXYD) * P2 + hq2);
-    gh2 = __ldg(met + (xi_halo ? mXYC : mC) * P2 + hq2);
-    gh3 = __ldg(met + (xi_halo ? mDivX : mDivY) * P2 + hq2);
+  for (int q = 0; q < V; ++q) {
+#pragma unroll
+    for (int d = 0; d < 7; ++d) { ap[d][q] = T(0); av[d][q] = T(0); }
+#pragma unroll
+    for (int d = 0; d < 4; ++d) { kp[d][q] = T(0); kv[d][q] = T(0); }
   }
   int slot = 0;
   uint32_t phase = 0;
   bool ok = true, failed = false;
-  const int bo = (ty + 3) * PW + tx + 4;           // own point in a box
-  const int to = ty * TX + tx;                     // own point in a tile
+  const int bo = (ty + 3) * PW + V * cx + 4;       // own points in a box
+  const int to = ty * TX + V * cx;                 // own points in a tile
+  const T k2 = -a.dt * a.inv_dxi;
   for (int m = kb - 3; m <= ke + 2; ++m) {
     const bool real = (m >= 0 && m < nr);
     const bool own = (m >= kb && m < ke);
     const bool bc = (m == 0 || m == nr - 1);
-    T r1 = T(0), r2 = T(0), part_p = T(0), part_v = T(0), facr_m = T(0);
     if (real) {
       const int o = m * plane + own0;
-      const long long plane_c2 = (long long)(face_c2 + m) * P2;
-      const bool do_halo = own && h_in && !bc;
-      // the gradient accumulator is read before the ring wait, so that its DRAM latency
-      // passes during the wait and the plane's arithmetic instead of stalling the store
-      const double gacc = (own && a.grad) ? a.grad[plane_c2 + p2] : 0.0;
       if (ok) {
         ok = mbar_wait(&bars[slot], phase, a.wc, kErrAdjointRing);
         if (ok) m_seen = m + 1;
       }
       const T* sb = reinterpret_cast<const T*>(slot_base(slot));
-      const T* rrow = reinterpret_cast<const T*>(slot_base(slot) + L::RAD_OFF);
-      const T invr = rrow[rInvR], inv_rho0 = rrow[rInvRho0], rho0 = rrow[rRho0], c2r = rrow[rC2Rho0];
-      facr_m = rrow[rFacR];
-      constexpr int PBs = (int)(L::P_BYTES / sizeof(T)), OBs = (int)(L::O_BYTES / sizeof(T));
-      const T* sc2 = reinterpret_cast<const T*>(slot_base(slot) + L::AUX);
-      const T c2own = tc2 ? sc2[bo] : T(0);
-      const T divv = (own && tdiv) ? sc2[(L::DIV_OFF - L::AUX) / sizeof(T) + to] : T(0);
-      T lqv[5], lwv[5];
+      const T* sc2 = reinterpret_cast<const T*>(slot_base(slot) + L::C2);
+      T rr[12];
 #pragma unroll
-      for (int f = 0; f < 5; ++f) { lqv[f] = T(0); lwv[f] = T(0); }
-      if (own) {
-        const int bf[4] = {kVxi, kVeta, kP, kRho};
+      for (int q = 0; q < 12; q += V) ldv(reinterpret_cast<const T*>(slot_base(slot) + L::RAD) + q, rr + q);
+      const T invr = rr[rInvR], inv_rho0 = rr[rInvRho0], rho0 = rr[rRho0];
+      T mP[V], mR[V], mRho[V], cc[V], e[V];        // mu of p, v_r, rho
+      ldv(own ? sb + L::PBOX / sizeof(T) + bo : sb + OBs + to, mP);
+      ldv(own ? sb + L::VR / sizeof(T) + to : sb + to, mR);
+      if (HAS_RHO) ldv(own ? sb + bo : sb + 2 * OBs + to, mRho);
+      if (tc2) ldv(own ? sc2 + bo : sc2 + to, cc);
+      T lP[V], lR[V], lRho[V];                     // lambda_q (the first stage's boxes hold it)
 #pragma unroll
-        for (int f = 0; f < 4; ++f) {
-          if (f == 3 && !has_rho) continue;
-          lqv[bf[f]] = sb[(2 * f) * PBs + bo];
-          lwv[bf[f]] = sb[(2 * f + 1) * PBs + bo];
+      for (int q = 0; q < V; ++q) {
+        lP[q] = mP[q];
+        lR[q] = mR[q];
+        mP[q] *= a.beta;
+        mR[q] *= a.beta;
+        if (HAS_RHO) { lRho[q] = mRho[q]; mRho[q] *= a.beta; }
+        const T c2rho0 = tc2 ? cc[q] * rho0 : rr[rC2Rho0];
+        e[q] = bc ? T(0) : -c2rho0 * mP[q] - (HAS_RHO ? rho0 * mRho[q] : T(0));
+      }
+      // banded radial transpose (rows 3 .. nr-4): plane m reaches the planes m-3 .. m+3
+      if (m >= 3 && m <= nr - 4) {
+        const T f = a.dt * rr[rFacR];
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          const T w1 = -f * inv_rho0 * mR[q], w2 = f * e[q];
+          ap[0][q] -= c3 * w1; ap[1][q] -= c2c * w1; ap[2][q] -= c1 * w1;
+          ap[4][q] += c1 * w1; ap[5][q] += c2c * w1; ap[6][q] += c3 * w1;
+          av[0][q] -= c3 * w2; av[1][q] -= c2c * w2; av[2][q] -= c1 * w2;
+          av[4][q] += c1 * w2; av[5][q] += c2c * w2; av[6][q] += c3 * w2;
         }
-        lqv[kVr] = sb[8 * PBs + to];
-        lwv[kVr] = sb[8 * PBs + OBs + to];
-      } else {
-        lqv[kP] = sb[to];
-        lwv[kP] = sb[OBs + to];
-        lqv[kVr] = sb[2 * OBs + to];
-        lwv[kVr] = sb[3 * OBs + to];
-        if (has_rho) { lqv[kRho] = sb[4 * OBs + to]; lwv[kRho] = sb[5 * OBs + to]; }
       }
-      T mu[5], mp[5];
-#pragma unroll
-      for (int f = 0; f < 5; ++f) {
-        mu[f] = lwv[f] + a.beta * lqv[f];
-        mp[f] = bc ? T(0) : mu[f];
-      }
-      const T c2rho0 = a.c2 ? c2own * rho0 : c2r;
-      const T e = -c2rho0 * mp[kP] - rho0 * mp[kRho];
-      r1 = -inv_rho0 * mp[kVr];
-      r2 = e;
       if (own) {
-        sX1[ty][tx + 3] = -invr * inv_rho0 * (gD * mp[kVxi] + gXYC * mp[kVeta]);
-        sX2[ty][tx + 3] = invr * gDivX * e;
-        sY1[ty + 3][tx] = -invr * inv_rho0 * (gXYD * mp[kVxi] + gC * mp[kVeta]);
-        sY2[ty + 3][tx] = invr * gDivY * e;
-        if (has_halo) {
-          T v1 = T(0), v2 = T(0);
-          if (do_halo) {
-            const int hb = (hj + 3) * PW + hi + 4;
-            const T hx = sb[1 * PBs + hb] + a.beta * sb[0 * PBs + hb];
-            const T hy = sb[3 * PBs + hb] + a.beta * sb[2 * PBs + hb];
-            const T hp = sb[5 * PBs + hb] + a.beta * sb[4 * PBs + hb];
-            const T hr = has_rho ? sb[7 * PBs + hb] + a.beta * sb[6 * PBs + hb] : T(0);
-            const T he = -(a.c2 ? sc2[hb] * rho0 : c2r) * hp - rho0 * hr;
-            v1 = -invr * inv_rho0 * (gh1 * hx + gh2 * hy);
-            v2 = invr * gh3 * he;
+        T* const ex = reinterpret_cast<T*>(smem + L::EX + (m & 1) * L::EX_BYTES);
+        T* const sX1 = ex;
+        T* const sX2 = ex + L::XB;
+        T* const sY1 = ex + 2 * L::XB;
+        T* const sY2 = ex + 2 * L::XB + L::YB;
+        T mX[V], mE[V], lX[V], lE[V];              // v_xi, v_eta
+        ldv(sb + R0 * PBs + bo, mX);
+        ldv(sb + (R0 + 1) * PBs + bo, mE);
+        {
+          const T f = -invr * inv_rho0;
+          T x1[V], x2[V], y1[V], y2[V];
+#pragma unroll
+          for (int q = 0; q < V; ++q) {
+            lX[q] = mX[q];
+            lE[q] = mE[q];
+            mX[q] *= a.beta;
+            mE[q] *= a.beta;
+            const T px = bc ? T(0) : mX[q], pe = bc ? T(0) : mE[q];
+            x1[q] = f * (gD[q] * px + gXYC[q] * pe);
+            x2[q] = invr * gDivX[q] * e[q];
+            y1[q] = f * (gXYD[q] * px + gC[q] * pe);
+            y2[q] = invr * gDivY[q] * e[q];
           }
-          if (xi_halo) { sX1[hj][hi + 3] = v1; sX2[hj][hi + 3] = v2; }
-          else { sY1[hj + 3][hi] = v1; sY2[hj + 3][hi] = v2; }
+          const int xo = ty * PW + V * cx + 4, yo = (ty + 3) * TX + V * cx;
+          stv(sX1 + xo, x1);
+          stv(sX2 + xo, x2);
+          stv(sY1 + yo, y1);
+          stv(sY2 + yo, y2);
         }
-        // pointwise terms, lw update, gradient
-        const T sig = rrow[rSigma];
-        T pw[5];
-        pw[kRho] = -rrow[rG0Rho0] * mp[kVr] - sig * mu[kRho];
-        pw[kVxi] = -invr * gTX * e;
-        pw[kVeta] = -invr * gTY * e;
-        pw[kVr] = T(2) * invr * e - rrow[rDRho0] * mp[kRho] + rrow[rRho0G0] * mp[kP] - sig * mu[kVr];
-        pw[kP] = -sig * mu[kP];
+        if (has_halo) {
+          T v1[V], v2[V];
 #pragma unroll
-        for (int f = 0; f < 5; ++f) {
-          const int s = g.slot[f];
-          if (s < 0) continue;
-          lw_face[fo(s) + o] = a.alpha * mu[f];
-          const T base = (a.keep ? lqv[f] : T(0)) + a.dt * pw[f];
-          if (f == kP) part_p = base;
-          else if (f == kVr) part_v = base;
-          else if (f == kRho) lo_face[fo(s) + o] = base;
-          else lqv[f] = base;                                  // v_xi, v_eta: 2-D part added below
+          for (int q = 0; q < V; ++q) { v1[q] = T(0); v2[q] = T(0); }
+          if (h_in && !bc) {
+            T hx[V], he[V], hp[V], hr[V], hc[V];
+            ldv(sb + R0 * PBs + hb, hx);
+            ldv(sb + (R0 + 1) * PBs + hb, he);
+            ldv(sb + L::PBOX / sizeof(T) + hb, hp);
+            if (HAS_RHO) ldv(sb + hb, hr);
+            if (tc2) ldv(sc2 + hb, hc);
+            const T f = -invr * inv_rho0 * a.beta, fe = -invr * a.beta;
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+              const T c2rho0 = tc2 ? hc[q] * rho0 : rr[rC2Rho0];
+              v1[q] = f * (gh1[q] * hx[q] + gh2[q] * he[q]);
+              v2[q] = fe * gh3[q] * (c2rho0 * hp[q] + (HAS_RHO ? rho0 * hr[q] : T(0)));
+            }
+          }
+          const int ho = xi_halo ? hj * PW + hi + 4 : (hj + 3) * TX + hi;
+          stv((xi_halo ? sX1 : sY1) + ho, v1);
+          stv((xi_halo ? sX2 : sY2) + ho, v2);
         }
-        if (a.grad) {
-          const T c = sqrt(c2rho0 * inv_rho0);
-          a.grad[plane_c2 + p2] = gacc + (double)(a.dt * (T(-2) * c * rho0 * divv) * mp[kP]);
+        // pointwise terms and the gradient
+        if (!a.first) {
+          const T* lq = sb + L::LQ / sizeof(T) + to;
+          if (HAS_RHO) ldv(lq, lRho);
+          ldv(lq + R0 * OBs, lX);
+          ldv(lq + (R0 + 1) * OBs, lE);
+          ldv(lq + (R0 + 2) * OBs, lR);
+          ldv(lq + (R0 + 3) * OBs, lP);
         }
-        if (m == 1 || m == 2 || m == nr - 3 || m == nr - 2) {
-          const int row = m <= 2 ? m - 1 : m - (nr - 3) + 2;
-          T* rbp = a.rb + (((long long)face * 4 + row) * 2) * P2 + p2;
-          rbp[0] = r1;
-          rbp[P2] = r2;
+        const T sig = rr[rSigma];
+        T orho[V], nrho[V];
+        T div[V];
+        double gacc[V];
+        if (tdiv) {
+          ldv(reinterpret_cast<const T*>(slot_base(slot) + L::DIV) + to, div);
+#pragma unroll
+          for (int q = 0; q < V; q += 2) ldv(reinterpret_cast<const double*>(slot_base(slot) + L::GRAD) + to + q, gacc + q);
         }
-        __syncthreads();
-        const T* x1 = &sX1[ty][tx + 3];
-        const T* x2 = &sX2[ty][tx + 3];
-        const T* y1 = &sY1[ty + 3][tx];
-        const T* y2 = &sY2[ty + 3][tx];
-        const T dx1 = c1 * (x1[1] - x1[-1]) + c2c * (x1[2] - x1[-2]) + c3 * (x1[3] - x1[-3]);
-        const T dx2 = c1 * (x2[1] - x2[-1]) + c2c * (x2[2] - x2[-2]) + c3 * (x2[3] - x2[-3]);
-        const T dy1 = c1 * (y1[TX] - y1[-TX]) + c2c * (y1[2 * TX] - y1[-2 * TX]) + c3 * (y1[3 * TX] - y1[-3 * TX]);
-        const T dy2 = c1 * (y2[TX] - y2[-TX]) + c2c * (y2[2 * TX] - y2[-2 * TX]) + c3 * (y2[3 * TX] - y2[-3 * TX]);
-        const T k2 = -a.dt * a.inv_dxi;
-        part_p += k2 * (dx1 + dy1);
-        lo_face[fo(sX) + o] = lqv[kVxi] + k2 * dx2;
-        lo_face[fo(sY) + o] = lqv[kVeta] + k2 * dy2;
-        // ghost-frame adjoints of the neighbour faces' values (W/E columns, S/N rows)
-        if ((i0 == 0 && tx < 3) || (i0 + TX == n && tx >= TX - 3)) {
-          const bool west = i0 == 0 && tx < 3;
-          const int c = west ? tx : TX + 3 + (tx - (TX - 3));  // x index of the ghost column
-          auto xv = [&](const T* row, int q) { return (q >= 0 && q < XW) ? row[q] : T(0); };
-          const T* r1p = &sX1[ty][0];
-          const T* r2p = &sX2[ty][0];
-          const T f1 = c1 * (xv(r1p, c + 1) - xv(r1p, c - 1)) + c2c * (xv(r1p, c + 2) - xv(r1p, c - 2)) + c3 * (xv(r1p, c + 3) - xv(r1p, c - 3));
-          const T f2 = c1 * (xv(r2p, c + 1) - xv(r2p, c - 1)) + c2c * (xv(r2p, c + 2) - xv(r2p, c - 2)) + c3 * (xv(r2p, c + 3) - xv(r2p, c - 3));
-          const int og = o - i + (west ? tx - 3 : n + (tx - (TX - 3)));
-          lo_face[fo(sP) + og] = k2 * f1;
-          lo_face[fo(sX) + og] = k2 * f2;
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          const T pr = bc ? T(0) : mR[q], pp = bc ? T(0) : mP[q];
+          T vr_ = T(2) * invr * e[q] + rr[rRho0G0] * pp - sig * mR[q];
+          if (HAS_RHO) {
+            vr_ -= rr[rDRho0] * (bc ? T(0) : mRho[q]);
+            orho[q] = (a.keep ? lRho[q] : T(0)) + a.dt * (-rr[rG0Rho0] * pr - sig * mRho[q]);
+            nrho[q] = a.alpha * mRho[q] + a.beta_next * orho[q];
+          }
+          ap[3][q] += (a.keep ? lP[q] : T(0)) - a.dt * sig * mP[q];
+          av[3][q] += (a.keep ? lR[q] : T(0)) + a.dt * vr_;
+          kp[3][q] = a.alpha * mP[q];
+          kv[3][q] = a.alpha * mR[q];
+          lX[q] = (a.keep ? lX[q] : T(0)) - a.dt * (invr * gTX[q] * e[q]);
+          lE[q] = (a.keep ? lE[q] : T(0)) - a.dt * (invr * gTY[q] * e[q]);
+          if (tdiv) gacc[q] += (double)(a.dt * (rho0 * div[q]) * pp);
         }
-        if ((j0 == 0 && ty < 3) || (j0 + TY == n && ty >= TY - 3)) {
-          const bool south = j0 == 0 && ty < 3;
-          const int r = south ? ty : TY + 3 + (ty - (TY - 3));  // y index of the ghost row
-          auto yv = [&](const T (*col)[TX], int q) { return (q >= 0 && q < YH) ? col[q][tx] : T(0); };
-          const T f1 = c1 * (yv(sY1, r + 1) - yv(sY1, r - 1)) + c2c * (yv(sY1, r + 2) - yv(sY1, r - 2)) + c3 * (yv(sY1, r + 3) - yv(sY1, r - 3));
-          const T f2 = c1 * (yv(sY2, r + 1) - yv(sY2, r - 1)) + c2c * (yv(sY2, r + 2) - yv(sY2, r - 2)) + c3 * (yv(sY2, r + 3) - yv(sY2, r - 3));
-          const int og = o + ((south ? ty - 3 : n + (ty - (TY - 3))) - j) * g.pitch;
-          lo_face[fo(sP) + og] = k2 * f1;
-          lo_face[fo(sY) + og] = k2 * f2;
+        if (tdiv) {
+          double* gp = a.grad + ((long long)face * nr + m) * P2 + p2;
+#pragma unroll
+          for (int q = 0; q < V; q += 2) stv(gp + q, gacc + q);
         }
+        if (HAS_RHO) {
+          stv(lo_face + sRho * vs + o, orho);
+          if (mu_face) stv(mu_face + sRho * vs + o, nrho);
+        }
+        // every thread is done with the slot and has written its exchange vectors
+        if (__syncthreads_or(!ok)) { failed = true; break; }
+        if (tid == 0 && loads && m_issued <= m_hi) issue(m_issued++, slot);
+        T w1[NV * V], w2[NV * V];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          ldv(sX1 + ty * PW + (cx + q) * V, w1 + q * V);
+          ldv(sX2 + ty * PW + (cx + q) * V, w2 + q * V);
+        }
+        T d1[V], d2[V], dy2[V];
+        {
+          T u[3][V], d[3][V];
+          const int yo = (ty + 3) * TX + V * cx;
+#pragma unroll
+          for (int r = 1; r <= 3; ++r) { ldv(sY1 + yo + r * TX, u[r - 1]); ldv(sY1 + yo - r * TX, d[r - 1]); }
+#pragma unroll
+          for (int q = 0; q < V; ++q)
+            d1[q] = c1 * (u[0][q] - d[0][q]) + c2c * (u[1][q] - d[1][q]) + c3 * (u[2][q] - d[2][q]);
+#pragma unroll
+          for (int r = 1; r <= 3; ++r) { ldv(sY2 + yo + r * TX, u[r - 1]); ldv(sY2 + yo - r * TX, d[r - 1]); }
+#pragma unroll
+          for (int q = 0; q < V; ++q)
+            dy2[q] = c1 * (u[0][q] - d[0][q]) + c2c * (u[1][q] - d[1][q]) + c3 * (u[2][q] - d[2][q]);
+        }
+        auto dxi = [&](const T* w, int c) {        // c = index into the window; zero past it
+          auto at = [&](int q) { return (q >= 0 && q < NV * V) ? w[q] : T(0); };
+          return c1 * (at(c + 1) - at(c - 1)) + c2c * (at(c + 2) - at(c - 2)) + c3 * (at(c + 3) - at(c - 3));
+        };
+        T nX[V], nE[V];
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          d1[q] += dxi(w1, 4 + q);
+          d2[q] = dxi(w2, 4 + q);
+          ap[3][q] += k2 * d1[q];
+          lX[q] += k2 * d2[q];
+          lE[q] += k2 * dy2[q];
+          nX[q] = a.alpha * mX[q] + a.beta_next * lX[q];
+          nE[q] = a.alpha * mE[q] + a.beta_next * lE[q];
+        }
+        stv(lo_face + sX * vs + o, lX);
+        stv(lo_face + sY * vs + o, lE);
+        if (mu_face) {
+          stv(mu_face + sX * vs + o, nX);
+          stv(mu_face + sY * vs + o, nE);
+        }
+        // ghost-frame adjoints of the neighbour faces' values (W/E columns, S/N rows); the
+        // exchange arrays are zero outside the face
+        if (i0 == 0 && cx == 0) {
+#pragma unroll
+          for (int c = 1; c <= 3; ++c) {
+            lo_face[sP * vs + o - 4 + c] = k2 * dxi(w1, c);
+            lo_face[sX * vs + o - 4 + c] = k2 * dxi(w2, c);
+          }
+        }
+        if (i0 + TX == n && cx == NT - 1) {
+#pragma unroll
+          for (int c = V + 4; c <= V + 6; ++c) {
+            lo_face[sP * vs + o - 4 + c] = k2 * dxi(w1, c);
+            lo_face[sX * vs + o - 4 + c] = k2 * dxi(w2, c);
+          }
+        }
+        const bool south = j0 == 0 && ty < 3, north = j0 + TY == n && ty >= TY - 3;
+        if (south || north) {
+#pragma unroll
+          for (int side = 0; side < 2; ++side) {
+            if (side == 0 ? !south : !north) continue;
+            const int r = side == 0 ? ty : ty + 6;           // exchange row of the ghost row
+            auto dy = [&](const T* y, int q) {
+              auto at = [&](int row) { return (row >= 0 && row < YH) ? y[row * TX + V * cx + q] : T(0); };
+              return c1 * (at(r + 1) - at(r - 1)) + c2c * (at(r + 2) - at(r - 2)) + c3 * (at(r + 3) - at(r - 3));
+            };
+            T f1[V], f2[V];
+#pragma unroll
+            for (int q = 0; q < V; ++q) { f1[q] = k2 * dy(sY1, q); f2[q] = k2 * dy(sY2, q); }
+            const int og = o + (side == 0 ? -3 : 3) * g.pitch;
+            stv(lo_face + sP * vs + og, f1);
+            stv(lo_face + sY * vs + og, f2);
+          }
+        }
+      } else {
+        if (__syncthreads_or(!ok)) { failed = true; break; }
+        if (tid == 0 && loads && m_issued <= m_hi) issue(m_issued++, slot);
       }
+      if (++slot == kAdjRing) { slot = 0; phase ^= 1; }
     }
-    // radial windows and the partial-output ring advance one plane
-    const bool band = real && m >= 3 && m <= nr - 4;
-    const T facr = band ? facr_m : T(0);
-#pragma unroll
-    for (int q = 0; q < 6; ++q) { w1[q] = w1[q + 1]; w2[q] = w2[q + 1]; }
-    w1[6] = facr * r1;
-    w2[6] = facr * r2;
-#pragma unroll
-    for (int q = 0; q < 3; ++q) { pp[q] = pp[q + 1]; pv[q] = pv[q + 1]; }
-    pp[3] = part_p;
-    pv[3] = part_v;
     const int pl = m - 3;
     if (pl >= kb && pl < ke) {
-      // (Dr^T R)_pl = sum_d a_d facr_{pl-d} R_{pl-d}, a_{-d} = -a_d; window index of pl-d is 3-d
-      const T rp = c1 * (w1[2] - w1[4]) + c2c * (w1[1] - w1[5]) + c3 * (w1[0] - w1[6]);
-      const T rv = c1 * (w2[2] - w2[4]) + c2c * (w2[1] - w2[5]) + c3 * (w2[0] - w2[6]);
+      if (pl < 7 || pl >= nr - 7) {
+        const bool low = pl < 7;
+        if (!low && pl == max(kb, nr - 7)) { one_sided(nr - 3, 0); one_sided(nr - 2, 1); }
+        const T* d = reinterpret_cast<const T*>(smem + L::ONE) + (size_t)tid * V;
+#pragma unroll
+        for (int row = 0; row < 2; ++row) {
+          const T b = low ? Coef<T>::bdy(1 + row, pl) : -Coef<T>::bdy(2 - row, nr - 1 - pl);
+          T r1[V], r2[V];
+          ldv(d + (2 * row) * L::NTH * V, r1);
+          ldv(d + (2 * row + 1) * L::NTH * V, r2);
+#pragma unroll
+          for (int q = 0; q < V; ++q) { ap[0][q] += b * r1[q]; av[0][q] += b * r2[q]; }
+        }
+      }
       const int op = pl * plane + own0;
-      lo_face[fo(sP) + op] = pp[0] + a.dt * rp;
-      lo_face[fo(sR) + op] = pv[0] + a.dt * rv;
+      stv(lo_face + sP * vs + op, ap[0]);
+      stv(lo_face + sR * vs + op, av[0]);
+      if (mu_face) {
+#pragma unroll
+        for (int q = 0; q < V; ++q) {
+          kp[0][q] += a.beta_next * ap[0][q];
+          kv[0][q] += a.beta_next * av[0][q];
+        }
+        stv(mu_face + sP * vs + op, kp[0]);
+        stv(mu_face + sR * vs + op, kv[0]);
+      }
     }
-    if (real) {
-      // every thread is done with this slot (and with the X/Y arrays): refill it
-      if (__syncthreads_or(!ok)) { failed = true; break; }
-      if (tid == 0 && loads && m_issued <= m_hi) issue(m_issued++, slot);
-      if (++slot == L::RING) { slot = 0; phase ^= 1; }
+    // the partial outputs advance one plane
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+#pragma unroll
+      for (int d = 0; d < 6; ++d) { ap[d][q] = ap[d + 1][q]; av[d][q] = av[d + 1][q]; }
+      ap[6][q] = T(0);
+      av[6][q] = T(0);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) { kp[d][q] = kp[d + 1][q]; kv[d][q] = kv[d + 1][q]; }
+      kp[3][q] = T(0);
+      kv[3][q] = T(0);
     }
   }
   // a wait gave up: wait (bounded) for the loads still in flight before the CTA exits
-  if (failed && tid == 0) mbar_drain(bars, L::RING, m_lo, m_seen, m_issued, a.wc.polls);
+  if (failed && tid == 0 && loads) mbar_drain(bars, kAdjRing, m_lo, m_seen, m_issued, a.wc.polls);
 }
 
-// The one-sided radial rows 1, 2 (onto planes 0..6) and nr-3, nr-2 (onto planes nr-7..nr-1)
-// of the radial transpose, added to p and v_r after adj_stage_kernel.
+// The gradient's last factor: grad holds sum dt rho0 div mu_p; dJ/dc = -2 c times that.
 template <typename T>
-__global__ void adj_rbdy_kernel(T* lout, const T* rb, const T* rad, Geom g, T dt) {
-  const int n = g.n, nr = g.nr;
-  const long long P2 = (long long)n * n;
+__global__ void grad_scale_kernel(double* grad, const T* c2, const T* radT, int nr, long long P2) {
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= 6 * 14 * P2) return;
-  const int face = (int)(idx / (14 * P2));
-  const int q = (int)((idx / P2) % 14);
-  const int p2 = (int)(idx % P2), i = p2 % n, j = p2 / n;
-  const bool low = q < 7;
-  const int pl = low ? q : nr - 14 + q;                      // planes 0..6 or nr-7..nr-1
-  T s1 = T(0), s2 = T(0);
-  for (int r = 0; r < 2; ++r) {
-    const int kk = low ? 1 + r : nr - 3 + r;
-    const int row = low ? r : 2 + r;
-    const T* rbp = rb + (((long long)face * 4 + row) * 2) * P2 + p2;
-    const T f = rad[rFacR * nr + kk];
-    const T b = low ? Coef<T>::bdy(kk, pl) : -Coef<T>::bdy(nr - 1 - kk, nr - 1 - pl);
-    s1 += f * b * rbp[0];
-    s2 += f * b * rbp[P2];
-  }
-  const long long o = g.at(pl, j, i);
-  lout[g.vol(0, face, g.slot[kP]) + o] += dt * s1;
-  lout[g.vol(0, face, g.slot[kVr]) + o] += dt * s2;
+  if (idx >= 6 * nr * P2) return;
+  const T* rr = radT + (size_t)((idx / P2) % nr) * 16;
+  const T c = sqrt(c2 ? c2[idx] : rr[rC2Rho0] * rr[rInvRho0]);
+  grad[idx] = -2.0 * (double)c * grad[idx];
 }
 
 // Transpose of the edge exchange, as a gather: every source-line point (the receiving face
@@ -413,8 +542,8 @@ __global__ void adj_rbdy_kernel(T* lout, const T* rb, const T* rad, Geom g, T dt
 // field scalar.  grid: x over u, y over (receiving face-edge, layer), z over planes; dynamic
 // shared memory: (mode 0 ? 2 : nf) x n values.
 template <typename T>
-__global__ void adj_edge_kernel(T* q, const T* __restrict__ wt, int span, const int* __restrict__ tspan, Geom g,
-                                int mode) {
+__global__ void adj_edge_kernel(T* q, T* mu, T beta, const T* __restrict__ wt, int span, const int* __restrict__ tspan,
+                                Geom g, int mode) {
   extern __shared__ __align__(16) unsigned char aesm[];
   T* const sg = reinterpret_cast<T*>(aesm);               // [field][t]
   __shared__ int s_lo, s_hi;
@@ -473,9 +602,16 @@ __global__ void adj_edge_kernel(T* q, const T* __restrict__ wt, int span, const 
     ax += __ldg(w + kind + j * n) * vv;
     ay += __ldg(w + 2 * kind + j * n) * vv;
   }
-  atomicAdd(q + g.vol(0, rt.src_face, g.slot[kP]) + src, ap);
-  atomicAdd(q + g.vol(0, rt.src_face, g.slot[kVxi]) + src, ax);
-  atomicAdd(q + g.vol(0, rt.src_face, g.slot[kVeta]) + src, ay);
+  const long long op = g.vol(0, rt.src_face, g.slot[kP]) + src, ox = g.vol(0, rt.src_face, g.slot[kVxi]) + src,
+                  oy = g.vol(0, rt.src_face, g.slot[kVeta]) + src;
+  atomicAdd(q + op, ap);
+  atomicAdd(q + ox, ax);
+  atomicAdd(q + oy, ay);
+  if (mu) {                                               // mu = alpha mu + beta lambda_q
+    atomicAdd(mu + op, beta * ap);
+    atomicAdd(mu + ox, beta * ax);
+    atomicAdd(mu + oy, beta * ay);
+  }
 }
 
 // FILTER_R^T for every stored field: u_m = sum over output planes k in [5, nr-6] of

@@ -22,7 +22,6 @@ static int adj_alloc(solar_ctx* c) {
     CK(cudaMemsetAsync(*p, 0, S, c->stream));
   }
   CK(cudaMalloc((void**)&b.grad, (size_t)6 * vol_compact(c) * sizeof(double)));
-  CK(cudaMalloc(&b.rb, (size_t)6 * 4 * 2 * c->g.n * c->g.n * c->esize));
   CK(cudaMalloc((void**)&b.tspan, c->ht.tspan.size() * sizeof(int)));
   CK(cudaMemcpy(b.tspan, c->ht.tspan.data(), c->ht.tspan.size() * sizeof(int), cudaMemcpyHostToDevice));
   // Edge weights transposed to the gather's order: wt[kind][row][j][u] is the coefficient
@@ -64,88 +63,85 @@ static int adj_reserve(void** p, size_t* have, size_t want) {
   return SOLAR_OK;
 }
 
+// Arguments of one transposed stage; as they stand, out = dt L^T(L) without the RK recursion.
 template <typename T>
 static AdjStageArgs<T> adj_args(solar_ctx* c, double dt) {
-  AdjStageArgs<T> a;
-  a.lout = nullptr;
-  a.lwout = nullptr;
-  a.rb = nullptr;
-  a.div = nullptr;
+  AdjStageArgs<T> a = {};
   a.c2 = (const T*)c->dt.c2;
-  a.grad = nullptr;
-  a.rad = (const T*)c->dt.rad;
   a.met = (const T*)c->dt.met;
   a.radT = (const T*)c->dt.radT;
   a.g = c->g;
-  a.alpha = T(0);
   a.beta = T(1);
   a.dt = (T)dt;
   a.inv_dxi = (T)(1.0 / c->ht.dxi);
-  a.keep = 0;
-  a.kchunk = 0;
+  a.first = 1;
   a.wc = wait_ctl(c, kInjAdjStage);
   return a;
 }
 
 static unsigned blocks_for(long long n, int threads) { return (unsigned)((n + threads - 1) / threads); }
 
-// L^T applied to buffer L (plus the pointwise and RK parts selected by `a`): the fused
-// transposed stage writes lambda_q and lambda_w to the partner buffers T1, T2 (inputs'
-// halos are read by neighbouring CTAs), the one-sided radial rows are added, the ghost
-// adjoints are scattered back, and the buffer pairs swap roles.
-template <typename T, int TX, int TY>
-static int launch_adj_stage(solar_ctx* c, AdjStageArgs<T>& a) {
-  using L = AdjLayout<T, TX, TY>;
+template <typename T, int TX, int TY, bool HAS_RHO>
+static int launch_adj_stage_t(solar_ctx* c, AdjStageArgs<T>& a) {
+  using L = AdjLayout<T, TX, TY, HAS_RHO>;
   AdjBuffers& b = c->adj;
-  if (!make_map(c, b.L, TX + 8, TY + 6, &a.mBq) || !make_map(c, b.LW, TX + 8, TY + 6, &a.mBw) ||
-      !make_map(c, b.L, TX, TY, &a.mTq) || !make_map(c, b.LW, TX, TY, &a.mTw) ||
-      (a.c2 && !make_compact_map(c, a.c2, TX + 8, TY + 6, &a.mC2)) || (a.grad && !make_compact_map(c, a.div, TX, TY, &a.mDiv)))
+  if (!make_fields_map(c, a.mu, TX + 8, TY + 6, HAS_RHO ? 3 : 2, &a.mB3) || !make_map(c, a.mu, TX + 8, TY + 6, &a.mB) ||
+      !make_map(c, a.mu, TX, TY, &a.mM) || !make_fields_map(c, a.mu, TX, TY, 2, &a.mM2) ||
+      !make_fields_map(c, b.L, TX, TY, c->g.nf, &a.mQ) ||
+      (a.c2 && (!make_compact_map(c, a.c2, TX + 8, TY + 6, &a.mC2) || !make_compact_map(c, a.c2, TX, TY, &a.mC2t))) ||
+      (a.grad && (!make_compact_map(c, a.div, TX, TY, &a.mDiv) || !make_compact_map(c, a.grad, TX, TY, &a.mGrad, true))))
     return fail(SOLAR_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-  if (!a.c2) a.mC2 = a.mTq;                       // unused
-  if (!a.grad) a.mDiv = a.mTq;
+  if (!a.c2) a.mC2 = a.mC2t = a.mM;               // unused
+  if (!a.grad) a.mDiv = a.mGrad = a.mM;
   static bool attr_set = false;
   static int resident = 1;
   if (!attr_set) {
-    CK(cudaFuncSetAttribute(adj_stage_kernel<T, TX, TY>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL));
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, adj_stage_kernel<T, TX, TY>, TX * TY, L::TOTAL));
+    CK(cudaFuncSetAttribute(adj_stage_kernel<T, TX, TY, HAS_RHO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, adj_stage_kernel<T, TX, TY, HAS_RHO>, L::NTH, L::TOTAL));
     resident = std::max(resident, 1);
     attr_set = true;
   }
   const Geom& g = c->g;
-  // Radial chunks: the count that minimises waves x planes per CTA, a chunk reading three
-  // planes more on either side (at 6 x 96^3 this picks 24-plane chunks, 2.92 waves: reverse
-  // sweep 4.6% faster than 20-plane chunks in 3.65 waves, in both precisions).
+  // Radial chunks: the count that minimises waves x (planes per CTA + 3): the three extra planes
+  // on either side move few bytes (us per reverse step at 6 x 96^3, float: + 3 850, + 6 862, + 9
+  // 1004; the same within 0.2% in double).
   const long long tiles = 6LL * (g.n / TX) * (g.n / TY);
   const long long slots = (long long)c->nsm * resident;
   int best = 1;
   long long best_cost = -1;
-  for (int nch = 1; nch <= std::max(1, g.nr / 8); ++nch) {
+  for (int nch = 1; nch <= g.nr; ++nch) {
     const long long kc = (g.nr + nch - 1) / nch;
-    const long long cost = ((tiles * nch + slots - 1) / slots) * (kc + 6);
+    const long long cost = ((tiles * nch + slots - 1) / slots) * (kc + 3);
     if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = nch; }
   }
   a.kchunk = (g.nr + best - 1) / best;
   dim3 grid((unsigned)((g.n / TX) * (g.n / TY)), (unsigned)((g.nr + a.kchunk - 1) / a.kchunk), 6);
-  adj_stage_kernel<T, TX, TY><<<grid, TX * TY, L::TOTAL, c->stream>>>(a);
+  CK(launch_pdl(adj_stage_kernel<T, TX, TY, HAS_RHO>, grid, dim3(TX / L::V, TY), L::TOTAL, c->stream, a));
   return SOLAR_OK;
 }
 
+template <typename T, int TX, int TY>
+static int launch_adj_stage(solar_ctx* c, AdjStageArgs<T>& a) {
+  return c->g.slot[kRho] >= 0 ? launch_adj_stage_t<T, TX, TY, true>(c, a) : launch_adj_stage_t<T, TX, TY, false>(c, a);
+}
+
+// One transposed stage on the buffers L (lambda_q) and LW (mu; not read in the first stage):
+// the fused kernel writes lambda_q and, unless the stage is the last one, the next mu to the
+// partner buffers T1, T2 (inputs' halos are read by neighbouring CTAs), the ghost adjoints
+// are scattered back into both, and the buffer pairs swap roles.
 template <typename T>
-static int enqueue_rhs_adjoint(solar_ctx* c, AdjStageArgs<T> a) {
+static int enqueue_rhs_adjoint(solar_ctx* c, AdjStageArgs<T> a, bool last) {
   AdjBuffers& b = c->adj;
   const Geom& g = c->g;
+  a.mu = (const T*)(a.first ? b.L : b.LW);
   a.lout = (T*)b.T1;
-  a.lwout = (T*)b.T2;
-  a.rb = (T*)b.rb;
-  a.wc = wait_ctl(c, kInjAdjStage);
+  a.muout = last ? nullptr : (T*)b.T2;
   if ((long long)g.nf * g.vs >= (1LL << 31))     // the kernel indexes one face's fields in 32 bits
     return fail(SOLAR_ERR_ARG, "grid too large for the adjoint (%lld values per face)", (long long)g.nf * g.vs);
   int rc = (g.n % 32 == 0) ? launch_adj_stage<T, 32, 8>(c, a) : launch_adj_stage<T, 16, 16>(c, a);
   if (rc) return rc;
-  adj_rbdy_kernel<T><<<blocks_for(6LL * 14 * g.n * g.n, 256), 256, 0, c->stream>>>((T*)b.T1, (const T*)b.rb,
-                                                                                   (const T*)c->dt.rad, g, a.dt);
   adj_edge_kernel<T><<<dim3(blocks_for(g.n, 128), 72, g.nr), 128, 2 * g.n * sizeof(T), c->stream>>>(
-      (T*)b.T1, (const T*)b.wt, b.wt_span, b.tspan, g, 0);
+      a.lout, a.muout, a.beta_next, (const T*)b.wt, b.wt_span, b.tspan, g, 0);
   CK(cudaGetLastError());
   std::swap(b.L, b.T1);
   std::swap(b.LW, b.T2);
@@ -171,7 +167,7 @@ static int enqueue_filter_adjoint(solar_ctx* c) {
         T1, L, g, KP);
   }
   adj_edge_kernel<T><<<dim3(blocks_for(g.n, 128), 72, g.nr), 128, g.nf * g.n * sizeof(T), c->stream>>>(
-      L, (const T*)c->adj.wt, c->adj.wt_span, c->adj.tspan, g, 1);
+      L, nullptr, T(0), (const T*)c->adj.wt, c->adj.wt_span, c->adj.tspan, g, 1);
   CK(cudaGetLastError());
   return SOLAR_OK;
 }
@@ -182,15 +178,16 @@ template <typename T>
 static int enqueue_step_adjoint(solar_ctx* c, const T* dstep, double* grad) {
   int rc;
   if ((rc = enqueue_filter_adjoint<T>(c))) return rc;
-  CK(cudaMemsetAsync(c->adj.LW, 0, (size_t)state_bytes(c), c->stream));
   const long long V6 = 6 * vol_compact(c);
   for (int s = 4; s >= 0; --s) {
     AdjStageArgs<T> a = adj_args<T>(c, c->desc.dt);
-    a.alpha = s == 0 ? T(0) : (T)kAlpha[s];
-    a.beta = (T)kBeta[s];
+    a.first = s == 4;
+    a.beta = s == 4 ? (T)kBeta[4] : T(1);
+    a.alpha = (T)kAlpha[s];
+    a.beta_next = s > 0 ? (T)kBeta[s - 1] : T(0);
     a.keep = 1;
     if (grad && dstep) { a.grad = grad; a.div = dstep + s * V6; }
-    if ((rc = enqueue_rhs_adjoint<T>(c, a))) return rc;
+    if ((rc = enqueue_rhs_adjoint<T>(c, a, s == 0))) return rc;
   }
   return SOLAR_OK;
 }
@@ -321,6 +318,9 @@ static int misfit_gradient_t(solar_ctx* c, int N, int K, int K2, const double* d
       t_adj += a;
     }
   }
+  grad_scale_kernel<T><<<blocks_for(V6, 256), 256, 0, c->stream>>>(b.grad, (const T*)c->dt.c2, (const T*)c->dt.radT, c->g.nr,
+                                                                  (long long)c->g.n * c->g.n);
+  CK(cudaGetLastError());
   // leave the state (and the clock) at the initial condition
   CK(cudaMemcpyAsync(c->A, ckpt, S, cudaMemcpyDeviceToDevice, c->stream));
   if (c->forcing) CK(cudaMemcpyAsync(c->force_clock, clk, CL, cudaMemcpyDeviceToDevice, c->stream));
@@ -426,9 +426,8 @@ int solar_gpu_rhs_adjoint(solar_ctx* c, const double* mu, double* out) {
   if (!mu || !out) return fail(SOLAR_ERR_ARG, "null array");
   if ((rc = adj_alloc(c))) return rc;
   if ((rc = upload_fields(c, c->adj.L, 0, mu, 5, kAllFields, 5))) return rc;
-  CK(cudaMemsetAsync(c->adj.LW, 0, (size_t)state_bytes(c), c->stream));
-  rc = c->fp32 ? enqueue_rhs_adjoint<float>(c, adj_args<float>(c, 1.0))
-               : enqueue_rhs_adjoint<double>(c, adj_args<double>(c, 1.0));
+  rc = c->fp32 ? enqueue_rhs_adjoint<float>(c, adj_args<float>(c, 1.0), true)
+               : enqueue_rhs_adjoint<double>(c, adj_args<double>(c, 1.0), true);
   if (rc) return rc;
   if ((rc = download_fields(c, c->adj.L, 0, out, 5, kAllFields, 5))) return rc;
   return check_device_error(c);

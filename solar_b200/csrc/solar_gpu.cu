@@ -138,10 +138,9 @@ struct DevTables {
 // Device arrays of the discrete adjoint, allocated on first use (nruns == 1 only).
 struct AdjBuffers {
   void* L = nullptr;        // lambda_q (padded state layout; frames hold ghost adjoints)
-  void* LW = nullptr;       // lambda_w
+  void* LW = nullptr;       // mu = lambda_w + beta lambda_q of the next transposed stage
   void* T1 = nullptr;       // filter-transpose scratch
   void* T2 = nullptr;
-  void* rb = nullptr;       // R1, R2 of the one-sided radial rows (planes 1, 2, nr-3, nr-2)
   int* tspan = nullptr;     // ghost-point range of every source position (transposed exchange)
   void* wt = nullptr;       // T [3][72][wt_span][n] edge weights in the gather's order
   int wt_span = 0;
@@ -334,17 +333,36 @@ static bool make_map(const solar_ctx* c, const void* base, int bx, int by, CUten
   return r == CUDA_SUCCESS;
 }
 
-// A compact six-zone field [face][k][j][i] (c^2, stored divergences) as a 3-D array:
-// x = i, y = j, z = face * nr + k; box bx x by x 1.
-static bool make_compact_map(const solar_ctx* c, const void* base, int bx, int by, CUtensorMap* m) {
+// 4-D view of a whole buffer: x, y as above, z = k, w = volume ((run*6 + face)*nf + slot); box
+// bx x by x 1 x nfields, the boxes of consecutive slots one after the other.
+static bool make_fields_map(const solar_ctx* c, const void* base, int bx, int by, int nfields, CUtensorMap* m) {
   auto enc = tensor_map_encoder();
   if (!enc) return false;
   const Geom& g = c->g;
+  cuuint64_t dims[4] = {(cuuint64_t)g.pitch, (cuuint64_t)g.rows, (cuuint64_t)g.nr, (cuuint64_t)g.nruns * 6 * g.nf};
+  cuuint64_t strides[3] = {(cuuint64_t)g.pitch * c->esize, (cuuint64_t)g.plane * c->esize, (cuuint64_t)g.vs * c->esize};
+  cuuint32_t box[4] = {(cuuint32_t)bx, (cuuint32_t)by, 1, (cuuint32_t)nfields};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(m, c->fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4,
+                   const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
+// A compact six-zone field [face][k][j][i] (c^2, stored divergences in the kernel
+// precision, the gradient in double) as a 3-D array: x = i, y = j, z = face * nr + k; box
+// bx x by x 1.
+static bool make_compact_map(const solar_ctx* c, const void* base, int bx, int by, CUtensorMap* m, bool in_double = false) {
+  auto enc = tensor_map_encoder();
+  if (!enc) return false;
+  const Geom& g = c->g;
+  const bool f32 = c->fp32 && !in_double;
+  const size_t esize = f32 ? 4 : 8;
   cuuint64_t dims[3] = {(cuuint64_t)g.n, (cuuint64_t)g.n, (cuuint64_t)6 * g.nr};
-  cuuint64_t strides[2] = {(cuuint64_t)g.n * c->esize, (cuuint64_t)g.n * g.n * c->esize};
+  cuuint64_t strides[2] = {(cuuint64_t)g.n * esize, (cuuint64_t)g.n * g.n * esize};
   cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = enc(m, c->fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
+  CUresult r = enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
                    const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS;
@@ -949,7 +967,7 @@ int solar_gpu_finalize(solar_ctx* c) {
                   c->dt.rad64, c->dt.vol2, c->dt.drw, c->dt.c2_64, c->dt.tanx, c->dt.gr};
   for (void* p : ptrs)
     if (p) cudaFree(p);
-  void* aptrs[] = {c->adj.L, c->adj.LW, c->adj.T1, c->adj.T2, c->adj.rb, c->adj.tspan, c->adj.wt, c->adj.grad, c->adj.ckpt, c->adj.ckpt2,
+  void* aptrs[] = {c->adj.L, c->adj.LW, c->adj.T1, c->adj.T2, c->adj.tspan, c->adj.wt, c->adj.grad, c->adj.ckpt, c->adj.ckpt2,
                    c->adj.div, c->adj.traces, c->adj.rec_off, c->adj.rec_w, c->adj.clk, c->split_items, c->split_slots,
                    c->force_clock, c->force_exy, c->force_samples, c->force_xy, c->force_r, c->norm_ring};
   for (void* p : aptrs)
