@@ -492,7 +492,7 @@ static int launch_stage_t(solar_ctx* c, StageArgs<T>& a, const void* qin) {
   using L = StageLayout<T, TX, TY, HAS_RHO>;
   if (!make_map(c, qin, TX + 8, TY + 6, &a.mP) || !make_map(c, qin, TX + 8, TY, &a.mX) ||
       !make_map(c, qin, TX, TY + 6, &a.mY) || !make_map(c, qin, TX, TY, &a.mO) ||
-      !make_map(c, c->W, TX, TY, &a.mW) || (a.c2 && !make_compact_map(c, a.c2, TX, TY, &a.mC2)))
+      !(L::QW_ONE ? make_fields_map(c, c->W, TX, TY, c->g.nf, &a.mW) : make_map(c, c->W, TX, TY, &a.mW)) || (a.c2 && !make_compact_map(c, a.c2, TX, TY, &a.mC2)))
     return fail(SOLAR_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   static bool attr_set = false;
   if (!attr_set) {
