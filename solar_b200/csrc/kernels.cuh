@@ -98,6 +98,23 @@ __device__ __forceinline__ void stv(T* p, const T* in) {
   *reinterpret_cast<VT*>(p) = v;
 }
 
+// N consecutive values (N * sizeof(T) = 4, 8 or 16 bytes) in one access.
+template <int N, typename T>
+__device__ __forceinline__ void ldn(const T* p, T* out) {
+  if constexpr (N * sizeof(T) == 16) ldv(p, out);
+  else if constexpr (N == 2) {
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    out[0] = v.x;
+    out[1] = v.y;
+  } else out[0] = *p;
+}
+template <int N, typename T>
+__device__ __forceinline__ void stn(T* p, const T* in) {
+  if constexpr (N * sizeof(T) == 16) stv(p, in);
+  else if constexpr (N == 2) *reinterpret_cast<float2*>(p) = make_float2(in[0], in[1]);
+  else *p = in[0];
+}
+
 // One 32-byte sector in a single 256-bit store (sm_100); p must be 32-byte aligned.
 __device__ __forceinline__ void st_sector(float* p, const float* v) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]),
@@ -520,13 +537,24 @@ struct StageLayout {
   static constexpr size_t TOTAL_C2 = C2 + RING * O_BYTES;
 };
 
-// Each thread owns V consecutive points of one row (V = 16 bytes / sizeof(T)), so the
-// CTA has (TX/V) x TY threads and every shared-memory access is a 16-byte vector.
+// Each thread owns V consecutive points of one row, so the CTA has (TX/V) x TY threads and
+// every shared-memory access is a vector (16 bytes but for the case below).
+// V = 2 in float on the 256-point tiles, which the small grids use: twice the warps shorten a
+// plane where few CTAs share an SM (us per step: 6 x 48^2 x 40 117 -> 108.5, 6 x 48^2 x 33 102 ->
+// 96; 6 x 96^3 477 -> 476.5), while one value per thread doubles the instructions (578 at 6 x
+// 96^3, 6 x 32^3 in double 84 -> 86).  The 64 x 8 tile keeps four (6 x 128^3: 927, with two 996).
+template <typename T, int TX, int TY>
+struct StageVec {
+  static constexpr int value = sizeof(T) == 4 && TX * TY == 256 ? 2 : Vec16<T>::V;
+  // a stated bound of one CTA lets that variant keep 156 registers instead of 128 (108.5 us
+  // against 112.7 at 6 x 48^2 x 40)
+  static constexpr int min_blocks = value == Vec16<T>::V ? 0 : 1;
+};
 template <typename T, int TX, int TY, int MODE_, bool HAS_RHO, bool FORCE = false>
-__global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __grid_constant__ StageArgs<T> a) {
+__global__ void __launch_bounds__((TX / StageVec<T, TX, TY>::value) * TY, StageVec<T, TX, TY>::min_blocks) stage_kernel(const __grid_constant__ StageArgs<T> a) {
   constexpr bool STORE_DIV = MODE_ >= 4;
   constexpr int MODE = MODE_ == 4 ? 1 : (MODE_ == 5 ? 0 : MODE_);
-  constexpr int V = Vec16<T>::V;
+  constexpr int V = StageVec<T, TX, TY>::value;
   constexpr int kTile = TileRing<T>::value;
   constexpr int NT = TX / V;
   constexpr int NV = (V + 8) / V;            // vectors covering box columns c .. c+V+7
@@ -595,14 +623,14 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
   const int ib = i0 + V * cx, j = j0 + ty;
   const int p2 = j * n + ib;
   T m_D[V], m_XYD[V], m_C[V], m_XYC[V], m_DivX[V], m_DivY[V], m_TX[V], m_TY[V];
-  ldv(a.met + mD * P2 + p2, m_D);
-  ldv(a.met + mXYD * P2 + p2, m_XYD);
-  ldv(a.met + mC * P2 + p2, m_C);
-  ldv(a.met + mXYC * P2 + p2, m_XYC);
-  ldv(a.met + mDivX * P2 + p2, m_DivX);
-  ldv(a.met + mDivY * P2 + p2, m_DivY);
-  ldv(a.met + mTX * P2 + p2, m_TX);
-  ldv(a.met + mTY * P2 + p2, m_TY);
+  ldn<V>(a.met + mD * P2 + p2, m_D);
+  ldn<V>(a.met + mXYD * P2 + p2, m_XYD);
+  ldn<V>(a.met + mC * P2 + p2, m_C);
+  ldn<V>(a.met + mXYC * P2 + p2, m_XYC);
+  ldn<V>(a.met + mDivX * P2 + p2, m_DivX);
+  ldn<V>(a.met + mDivY * P2 + p2, m_DivY);
+  ldn<V>(a.met + mTX * P2 + p2, m_TX);
+  ldn<V>(a.met + mTY * P2 + p2, m_TY);
   const T c1 = Coef<T>::drp(1), c2 = Coef<T>::drp(2), c3 = Coef<T>::drp(3);
   if (tid == 0) {
     for (int q = 0; q < kLead + kTile; ++q) mbar_init(&barL[q], 1);
@@ -625,7 +653,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
   }
 
   T f_xy[V];
-  if (FORCE) ldv(a.force + (long long)face * P2 + p2, f_xy);
+  if (FORCE) ldn<V>(a.force + (long long)face * P2 + p2, f_xy);
   const long long own = g.at(0, j, ib);
   T* outS[5];
   T* qwS[5];
@@ -663,8 +691,8 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
       for (int s = 0; s < 6; ++s)
 #pragma unroll
         for (int q = 0; q < V; ++q) { pw[s][q] = pw[s + 1][q]; vw[s][q] = vw[s + 1][q]; }
-      ldv(bp + pc + 4, pw[6]);
-      ldv(reinterpret_cast<const T*>(lead(slot_q) + L::P_BYTES) + oc, vw[6]);
+      ldn<V>(bp + pc + 4, pw[6]);
+      ldn<V>(reinterpret_cast<const T*>(lead(slot_q) + L::P_BYTES) + oc, vw[6]);
       if (++slot_q == kLead) { slot_q = 0; phase_q ^= 1; }
     }
     if (ok && !mbar_wait(&barT[slot_t], phase_t, a.wc, kErrStageTile)) { ok = false; tile_fail = true; }
@@ -675,24 +703,24 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
     // xi windows of p and v_xi; eta columns of p and v_eta
     T wp[NV * V], wx[NV * V];
 #pragma unroll
-    for (int m = 0; m < NV; ++m) { ldv(sp + pc + m * V, wp + m * V); ldv(sx + xc + m * V, wx + m * V); }
+    for (int m = 0; m < NV; ++m) { ldn<V>(sp + pc + m * V, wp + m * V); ldn<V>(sx + xc + m * V, wx + m * V); }
     T pu[3][V], pd[3][V], yu[3][V], yd[3][V], vyo[V];
 #pragma unroll
     for (int d = 1; d <= 3; ++d) {
-      ldv(sp + pc + 4 + d * PW, pu[d - 1]);
-      ldv(sp + pc + 4 - d * PW, pd[d - 1]);
-      ldv(sy + yc + d * TX, yu[d - 1]);
-      ldv(sy + yc - d * TX, yd[d - 1]);
+      ldn<V>(sp + pc + 4 + d * PW, pu[d - 1]);
+      ldn<V>(sp + pc + 4 - d * PW, pd[d - 1]);
+      ldn<V>(sy + yc + d * TX, yu[d - 1]);
+      ldn<V>(sy + yc - d * TX, yd[d - 1]);
     }
-    ldv(sy + yc, vyo);
+    ldn<V>(sy + yc, vyo);
     T rho[V], qwv[5][V];
-    if (HAS_RHO && MODE != 3) ldv(reinterpret_cast<const T*>(tb + L::X_BYTES + L::Y_BYTES) + oc, rho);
+    if (HAS_RHO && MODE != 3) ldn<V>(reinterpret_cast<const T*>(tb + L::X_BYTES + L::Y_BYTES) + oc, rho);
     if (MODE == 0)
 #pragma unroll
       for (int f = 0; f < 5; ++f)
         if (f != kRho || HAS_RHO) {
           const int sl = HAS_RHO ? f : f - 1;
-          ldv(reinterpret_cast<const T*>(tb + L::X_BYTES + L::Y_BYTES + (QOFF + sl) * L::O_BYTES) + oc, qwv[f]);
+          ldn<V>(reinterpret_cast<const T*>(tb + L::X_BYTES + L::Y_BYTES + (QOFF + sl) * L::O_BYTES) + oc, qwv[f]);
         }
     const T* sc2 = reinterpret_cast<const T*>(smem + L::C2 + slot_t * L::O_BYTES) + oc;
     // The plane's radial coefficients come with its ring slot, every thread reading the same
@@ -702,7 +730,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
     // 128^3 in float 149.2 -> 146.6; read word by word at their uses 150).
     T rr[12];
 #pragma unroll
-    for (int m = 0; m < 12; m += V) ldv(reinterpret_cast<const T*>(tb + L::RAD) + m, rr + m);
+    for (int m = 0; m < 12; m += Vec16<T>::V) ldv(reinterpret_cast<const T*>(tb + L::RAD) + m, rr + m);
     const T facr = rr[rFacR], invr = rr[rInvR];
     T frc = T(0);
     if (FORCE) frc = __ldg(a.force_r + k);
@@ -760,18 +788,18 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
       }
     }
     const long long kp = (long long)k * g.plane;
-    if (STORE_DIV) stv(a.divout + ((long long)face * nr + k) * P2 + p2, dvv);
+    if (STORE_DIV) stn<V>(a.divout + ((long long)face * nr + k) * P2 + p2, dvv);
     if (MODE == 3) {
-      stv(outS[kVxi] + kp, o0);
-      stv(outS[kVeta] + kp, o1);
-      stv(outS[kVr] + kp, o2);
-      stv(outS[kP] + kp, o3);
+      stn<V>(outS[kVxi] + kp, o0);
+      stn<V>(outS[kVeta] + kp, o1);
+      stn<V>(outS[kVr] + kp, o2);
+      stn<V>(outS[kP] + kp, o3);
     } else if (MODE == 2) {
-      if (HAS_RHO) stv(outS[kRho] + kp, r_rho);
-      stv(outS[kVxi] + kp, r_vx);
-      stv(outS[kVeta] + kp, r_ve);
-      stv(outS[kVr] + kp, r_vr);
-      stv(outS[kP] + kp, r_p);
+      if (HAS_RHO) stn<V>(outS[kRho] + kp, r_rho);
+      stn<V>(outS[kVxi] + kp, r_vx);
+      stn<V>(outS[kVeta] + kp, r_ve);
+      stn<V>(outS[kVr] + kp, r_vr);
+      stn<V>(outS[kP] + kp, r_p);
     } else {
       // BC_RHS (bc_acoustic_wave.f90:14-34) then SPONGE (sponge.f90:40-50)
       const bool bc = (k == 0 || k == nr - 1);
@@ -787,8 +815,8 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) stage_kernel(const __
           w[q] = (MODE == 1) ? dt * r : fma(alpha, qwv[f][q], dt * r);
           o[q] = fma(beta, w[q], qv[q]);
         }
-        if (MODE == 1 || a.store_w) stv(qwS[f] + kp, w);
-        stv(outS[f] + kp, o);
+        if (MODE == 1 || a.store_w) stn<V>(qwS[f] + kp, w);
+        stn<V>(outS[f] + kp, o);
       };
       if (HAS_RHO) update(kRho, rho, r_rho, true);
       update(kVxi, vxv, r_vx, false);

@@ -505,19 +505,17 @@ static int launch_stage_t(solar_ctx* c, StageArgs<T>& a, const void* qin) {
   const int ntiles = stage_tile_count(a.tsel, c->g.n / TX, c->g.n / TY);
   if (ntiles <= 0) return SOLAR_OK;                // no interior tiles at this size
   const int nk = c->g.k1 - c->g.k0, volumes = launched_runs(c, a.runs) * c->g.nface;
-  if (a.kchunk <= 0) {
-    static int resident[2] = {0, 0};               // CTAs per SM without / with the c^2 boxes
-    int& res = resident[a.c2 ? 1 : 0];
-    if (!res) {
-      int r = 1;
-      CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, stage_kernel<T, TX, TY, MODE, HAS_RHO, FORCE>,
-                                                       TX / Vec16<T>::V * TY, smem));
-      res = std::max(r, 1);
-    }
-    a.kchunk = plan_planes(ntiles, volumes, nk, (long long)c->nsm * res, c->fp32);
+  static int resident[2] = {0, 0};                 // CTAs per SM without / with the c^2 boxes
+  int& res = resident[a.c2 ? 1 : 0];
+  if (!res) {
+    int r = 1;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&r, stage_kernel<T, TX, TY, MODE, HAS_RHO, FORCE>,
+                                                     TX / StageVec<T, TX, TY>::value * TY, smem));
+    res = std::max(r, 1);
   }
+  if (a.kchunk <= 0) a.kchunk = plan_planes(ntiles, volumes, nk, (long long)c->nsm * res, c->fp32);
   dim3 grid(ntiles, (nk + a.kchunk - 1) / a.kchunk, volumes);
-  CK(launch_pdl(stage_kernel<T, TX, TY, MODE, HAS_RHO, FORCE>, grid, dim3(TX / Vec16<T>::V, TY), smem, c->stream, a));
+  CK(launch_pdl(stage_kernel<T, TX, TY, MODE, HAS_RHO, FORCE>, grid, dim3(TX / StageVec<T, TX, TY>::value, TY), smem, c->stream, a));
   return SOLAR_OK;
 }
 
