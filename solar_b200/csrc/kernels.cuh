@@ -359,6 +359,7 @@ __global__ void __launch_bounds__(384, (EdgeMinBlocks<T>::value)) edge_kernel(co
   int ns = 1;                                            // ring slot of plane kk + 1 ...
   uint32_t np = 0;                                       // ... and the parity of its phase
   for (; kk < kc; ++kk) {
+    if (kk == kc - release_planes(kc)) release_dependents();
     if (tid == 0 && ok && !a.wc.no_loads && kk + kEdgeDepth < kc) issue(kk + kEdgeDepth, ws);
     ws = ws + 1 == kEdgeRing ? 0 : ws + 1;
     if (ns == 0) np ^= 1;
@@ -683,6 +684,7 @@ __global__ void __launch_bounds__((TX / StageVec<T, TX, TY>::value) * TY, StageV
   int lead_fail = 0x7fffffff;
   int k = kb;
   for (; k < ke; ++k) {
+    if (k == ke - release_planes(ke - kb)) release_dependents();
     const int ks = clampk(k);
     for (; mq <= ks + 6; ++mq) {
       if (ok && !mbar_wait(&barL[slot_q], phase_q, a.wc, kErrStageLead)) { ok = false; lead_fail = mq; }
@@ -987,6 +989,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 
     for (int u = 0; u < 11; ++u) {
       const int k = kb + u;
       if (k >= ke) break;
+      if (k == ke - release_planes(ke - ks)) release_dependents();
       const bool got = mbar_wait(&bars[slot], phase, a.wc, kErrFilterRing);
       const T* bx = reinterpret_cast<const T*>(smem + slot * L::P_BYTES);
       T* t1 = reinterpret_cast<T*>(smem + kFiltRing * L::P_BYTES + (k & 1) * L::S_BYTES);

@@ -134,9 +134,19 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
 // starts as its predecessor's last CTAs exit, before that grid has fully completed; it must
 // call grid_dependency_wait() before it reads anything the predecessor (or an earlier
 // kernel) wrote and before it writes anything, and only constant tables may be read before
-// that.  (No kernel here triggers its successor earlier: successor CTAs waiting on SMs during
-// a multi-wave stage kernel's last wave cost the FP32 step 1.5%.)
+// that.  The stepping kernels call release_dependents() when a CTA comes to its last planes: the
+// next kernel's CTAs start once every CTA has done so (or has exited), so they take only slots
+// that this grid has left for good, and their launch and prologue pass while the last planes
+// are computed.  One plane before the end for short chunks, two for longer ones (us per step
+// without, one, two: 6 x 48^2 x 40 108.5, 102.3, 110; 6 x 16^2 x 24 55, 46, 53; 6 x 64^3 in
+// double 361, 352, 349; 6 x 80^2 x 50 with a source 449, 437, 430; 6 x 128^3 923, 922, 920).
+// Released at a CTA's start instead, the waiting CTAs crowd onto few SMs or take the slots of a
+// last wave (6 x 48^2 x 40 115, 6 x 128^3 +1.5%).
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+__device__ __forceinline__ void release_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Planes before the end of a march of n planes at which it releases the next kernel.
+__device__ __forceinline__ int release_planes(int n) { return n > 6 ? 2 : 1; }
 
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
