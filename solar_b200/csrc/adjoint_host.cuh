@@ -334,7 +334,13 @@ static int misfit_gradient_t(solar_ctx* c, int N, int K, int K2, const double* d
     times[2] = t_adj;
   }
   if (grad_c) {
-    CK(cudaMemcpyAsync(grad_c, b.grad, (size_t)V6 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    const size_t bytes = (size_t)V6 * sizeof(double);
+    if (bytes >= 8u << 20 && stage_pageable(grad_c, bytes)) {
+      Staged st(c);
+      if ((rc = st.out(grad_c, b.grad, bytes)) || (rc = st.finish())) return rc;
+    } else {
+      CK(cudaMemcpyAsync(grad_c, b.grad, bytes, cudaMemcpyDeviceToHost, c->stream));
+    }
     CK(cudaStreamSynchronize(c->stream));
   }
   if (lambda0) return download_fields(c, c->adj.L, 0, lambda0, 5, kAllFields, 5);

@@ -164,6 +164,9 @@ struct AdjBuffers {
 
 using namespace solar;
 
+constexpr int kStageBlocks = 8;
+constexpr size_t kStageBytes = 4u << 20;
+
 struct solar_ctx {
   solar_desc desc;
   HostTables ht;
@@ -201,6 +204,9 @@ struct solar_ctx {
   float* pin32 = nullptr;
   cudaEvent_t xev[2] = {};
   std::unique_ptr<HostPool> pool;
+  // Pageable arrays of the caller move through kStageBlocks pinned blocks (on first use).
+  char* pin_stage = nullptr;
+  cudaEvent_t sev[kStageBlocks] = {};
   AdjBuffers adj;
   int forcing = 0;             // SOLAR_FORCING_*
   int force_nstep = 0, force_nt = 0;
@@ -776,14 +782,24 @@ static void drop_batch_graphs(solar_ctx* c) {
 // ---------------------------------------------------------------- transfers
 static long long vol_compact(const solar_ctx* c) { return (long long)c->g.n * c->g.n * c->g.nr; }
 
+// The context's host threads, on first use.
+static int ensure_pool(solar_ctx* c) {
+  if (c->pool) return SOLAR_OK;
+  try {
+    c->pool.reset(new HostPool(host_threads()));
+  } catch (const std::exception& e) {
+    return fail(SOLAR_ERR_NOMEM, "host threads: %s", e.what());
+  }
+  return SOLAR_OK;
+}
+
 // FP32 transfers: the pinned blocks, their events and the host threads, on first use.
 static int ensure_pin32(solar_ctx* c) {
   if (c->pin32) return SOLAR_OK;
   const size_t bytes = (size_t)2 * vol_compact(c) * sizeof(float);
   CK(cudaHostAlloc((void**)&c->pin32, bytes, cudaHostAllocDefault));
   for (auto& e : c->xev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  c->pool.reset(new HostPool(host_threads()));
-  return SOLAR_OK;
+  return ensure_pool(c);
 }
 
 // The slice [lo, hi) of n items that host thread t of p handles.
@@ -791,6 +807,100 @@ static void slice(long long n, int t, int p, long long* lo, long long* hi) {
   *lo = n * t / p;
   *hi = n * (t + 1) / p;
 }
+
+// Whether an array of the caller, moved in volumes of `bytes`, goes through the pinned blocks:
+// pageable memory in volumes of at least 1 MiB.  The driver moves such arrays through a staging
+// buffer of its own with one thread, which also takes the page faults of a fresh result array
+// (COMPUTE_RHS at 6 x 64^3 in double, 63 MB out into fresh memory: 16.2 ms, now 6.3; at 6 x 96^3
+// 50 ms, now 18; a pageable state in at 6 x 96^3 19.4 ms, now 7.0).  Smaller volumes do not
+// repay waking the threads (6 x 48^3, 0.9 MB each: the same 3.2 ms).
+static bool stage_pageable(const void* p, size_t bytes) {
+  if (bytes < (1u << 20)) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return false; }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
+static int ensure_stage(solar_ctx* c) {
+  if (c->pin_stage) return SOLAR_OK;
+  int rc;
+  if ((rc = ensure_pool(c))) return rc;
+  for (auto& e : c->sev)
+    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  CK(cudaHostAlloc((void**)&c->pin_stage, kStageBlocks * kStageBytes, cudaHostAllocDefault));
+  return SOLAR_OK;
+}
+
+// Copies between the device and a pageable array, on the context's stream, through the pinned
+// blocks in order: out() enqueues a block's copy off the device and, when every block is in
+// use, waits for the older half and lets the host threads copy it on in one go (waking them
+// costs as much as copying a megabyte); finish() drains the rest.  in() lets the threads fill a
+// block (once its last copy is done) and enqueues its copy.  The device side is stream-ordered,
+// so the caller may enqueue kernels that reuse it at once.
+class Staged {
+ public:
+  explicit Staged(solar_ctx* c) : c_(c) {}
+  int out(void* host, const void* dev, size_t bytes) {
+    int rc;
+    if ((rc = ensure_stage(c_))) return rc;
+    for (size_t o = 0; o < bytes; o += kStageBytes) {
+      if (head_ - tail_ == kStageBlocks && (rc = drain(kStageBlocks / 2))) return rc;
+      const int s = (int)(head_ % kStageBlocks);
+      const size_t n = std::min(kStageBytes, bytes - o);
+      CK(cudaMemcpyAsync(block(s), (const char*)dev + o, n, cudaMemcpyDeviceToHost, c_->stream));
+      CK(cudaEventRecord(c_->sev[s], c_->stream));
+      host_[s] = (char*)host + o;
+      len_[s] = n;
+      ++head_;
+    }
+    return SOLAR_OK;
+  }
+  int finish() {
+    int rc;
+    while (tail_ < head_)
+      if ((rc = drain((int)std::min<long long>(kStageBlocks / 2, head_ - tail_)))) return rc;
+    return SOLAR_OK;
+  }
+  int in(void* dev, const void* host, size_t bytes) {
+    int rc;
+    if ((rc = ensure_stage(c_))) return rc;
+    for (size_t o = 0; o < bytes; o += kStageBytes) {
+      const int s = (int)(head_ % kStageBlocks);
+      const size_t n = std::min(kStageBytes, bytes - o);
+      if (head_ >= kStageBlocks) CK(cudaEventSynchronize(c_->sev[s]));
+      HostPool& pool = *c_->pool;
+      pool.run([&](int t) { copy_slice(block(s), (const char*)host + o, n, t, pool.size()); });
+      CK(cudaMemcpyAsync((char*)dev + o, block(s), n, cudaMemcpyHostToDevice, c_->stream));
+      CK(cudaEventRecord(c_->sev[s], c_->stream));
+      ++head_;
+    }
+    return SOLAR_OK;
+  }
+
+ private:
+  char* block(int s) { return c_->pin_stage + (size_t)s * kStageBytes; }
+  int drain(int count) {                                   // the oldest `count` blocks
+    CK(cudaEventSynchronize(c_->sev[(tail_ + count - 1) % kStageBlocks]));
+    HostPool& pool = *c_->pool;
+    pool.run([&](int t) {
+      for (int q = 0; q < count; ++q) {
+        const int s = (int)((tail_ + q) % kStageBlocks);
+        copy_slice(host_[s], block(s), len_[s], t, pool.size());
+      }
+    });
+    tail_ += count;
+    return SOLAR_OK;
+  }
+  static void copy_slice(char* dst, const char* src, size_t n, int t, int p) {
+    long long lo, hi;
+    slice((long long)n, t, p, &lo, &hi);
+    std::memcpy(dst + lo, src + lo, (size_t)(hi - lo));
+  }
+  solar_ctx* c_;
+  char* host_[kStageBlocks] = {};
+  size_t len_[kStageBlocks] = {};
+  long long head_ = 0, tail_ = 0;
+};
 
 // FP32 context: each compact volume is rounded to float on the host (round to nearest even,
 // as the device conversion does, so the stored state is the same bit for bit) into one of
@@ -837,6 +947,9 @@ static int upload_fields(solar_ctx* c, void* buf, int run, const double* host, i
                          const int* fields, int nfields_h) {
   if (c->fp32) return upload_fields32(c, buf, run, host, nh, fields, nfields_h);
   const long long V = vol_compact(c);
+  const size_t bytes = (size_t)V * sizeof(double);
+  const bool staged = stage_pageable(host, bytes);
+  Staged st(c);
   const int threads = 256;
   const int blocks = (int)((V + threads - 1) / threads);
   for (int z = 0; z < 6; ++z)
@@ -844,8 +957,13 @@ static int upload_fields(solar_ctx* c, void* buf, int run, const double* host, i
       const int f = fields[m];
       const int s = c->g.slot[f];
       if (s < 0) continue;
-      CK(cudaMemcpyAsync(c->stage64, host + ((long long)z * nh + m) * V, V * sizeof(double),
-                         cudaMemcpyHostToDevice, c->stream));
+      const double* src = host + ((long long)z * nh + m) * V;
+      int rc;
+      if (staged) {
+        if ((rc = st.in(c->stage64, src, bytes))) return rc;
+      } else {
+        CK(cudaMemcpyAsync(c->stage64, src, bytes, cudaMemcpyHostToDevice, c->stream));
+      }
       const long long off = c->g.vol(run, z, s);
       if (c->fp32) unpack_kernel<float><<<blocks, threads, 0, c->stream>>>(c->stage64, (float*)buf + off, c->g);
       else unpack_kernel<double><<<blocks, threads, 0, c->stream>>>(c->stage64, (double*)buf + off, c->g);
@@ -857,6 +975,10 @@ static int upload_fields(solar_ctx* c, void* buf, int run, const double* host, i
 static int download_fields(solar_ctx* c, const void* buf, int run, double* host, int nh,
                            const int* fields, int nfields_h) {
   const long long V = vol_compact(c);
+  const size_t bytes = (size_t)V * sizeof(double);
+  const bool staged = stage_pageable(host, bytes);
+  Staged st(c);
+  int rc;
   const int threads = 256;
   const int blocks = (int)((V + threads - 1) / threads);
   for (int z = 0; z < 6; ++z)
@@ -871,8 +993,13 @@ static int download_fields(solar_ctx* c, const void* buf, int run, double* host,
       if (c->fp32) pack_kernel<float><<<blocks, threads, 0, c->stream>>>((const float*)buf + c->g.vol(run, z, s), c->stage64, c->g);
       else pack_kernel<double><<<blocks, threads, 0, c->stream>>>((const double*)buf + c->g.vol(run, z, s), c->stage64, c->g);
       CK(cudaGetLastError());
-      CK(cudaMemcpyAsync(dst, c->stage64, V * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+      if (staged) {
+        if ((rc = st.out(dst, c->stage64, bytes))) return rc;
+      } else {
+        CK(cudaMemcpyAsync(dst, c->stage64, bytes, cudaMemcpyDeviceToHost, c->stream));
+      }
     }
+  if ((rc = st.finish())) return rc;
   CK(cudaStreamSynchronize(c->stream));
   return SOLAR_OK;
 }
@@ -974,7 +1101,10 @@ int solar_gpu_finalize(solar_ctx* c) {
     if (e) cudaEventDestroy(e);
   for (auto& e : c->xev)
     if (e) cudaEventDestroy(e);
+  for (auto& e : c->sev)
+    if (e) cudaEventDestroy(e);
   if (c->pin32) cudaFreeHost(c->pin32);
+  if (c->pin_stage) cudaFreeHost(c->pin_stage);
   c->pool.reset();
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
