@@ -16,8 +16,8 @@
 //              values are the adjoints of the neighbour faces' ghost values;
 //   adj_edge   the transpose of the edge exchange: each source-line point gathers the ghost
 //              adjoints that used it, with the same folded coefficients.
-// FILTER_EXP^T is the radial transpose, then eta, then xi, each with its ghost-frame
-// adjoints, then the same scatter.
+// FILTER_EXP^T runs fused (adj_filter_kernel), its ghost-frame adjoints in a small kernel of
+// their own, then the same scatter.
 #pragma once
 
 #include "kernels.cuh"
@@ -614,145 +614,262 @@ __global__ void adj_edge_kernel(T* q, T* mu, T beta, const T* __restrict__ wt, i
   }
 }
 
-// FILTER_R^T for every stored field: u_m = sum over output planes k in [5, nr-6] of
-// fr_{|k-m|} lam_k (the end planes of the forward output are constant zeros).  One thread
-// per (field volume, j, i) column marches the planes with an 11-deep register queue, so
-// lam is read once.
-template <typename T>
-__global__ void adj_filter_r_kernel(const T* lam, T* u, Geom g) {
+// FILTER_EXP^T of one field on the face interior, fused.  The transpose is radial^T, then eta^T,
+// then xi^T; the three act along different axes, so they commute and the radial one can come
+// last, on a register queue as in filter_kernel: per plane the xi and eta filters with zero
+// halos (the tensor map covers the interior only, so the load fills them), then the 11-point
+// radial filter over the planes [5, nr-6] (the forward output is zero outside them).  Tiles,
+// threads, ring and work split are those of filter_kernel, and so is what bounds it.  us per
+// launch at 6 x 96^3 in double / float: 116 / 54, with adj_ghost_kernel's 42 / 29 beside it (as a
+// radial pass over the whole buffer and a plane-marching xi/eta pass with plain loads, ghost
+// adjoints included, 117 + 170 / 52 + 67; with a branch around the zero planes 134 / 69).
+template <typename T, int TX, int TY, int R>
+__global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 ? 4 : 1) adj_filter_kernel(const __grid_constant__ FilterArgs<T> a) {
+  constexpr int V = Vec16<T>::V, NT = TX / V, NY = TY / R, NV = (V + 8) / V, PW = TX + 8, NP = V / 2;
+  constexpr bool PAIRS = sizeof(T) == 4;
+  using L = FilterLayout<T, TX, TY>;
+  extern __shared__ __align__(128) unsigned char smem[];
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR);
+  const Geom& g = a.g;
   const int n = g.n, nr = g.nr;
-  const long long P = (long long)n * n;
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (long long)g.nruns * 6 * g.nf * P) return;
-  const long long vsel = idx / P;                      // (run*6 + face)*nf + slot
-  const int p2 = (int)(idx % P), i = p2 % n, j = p2 / n;
-  const T* L = lam + vsel * g.vs + g.at(0, j, i);
-  T* U = u + vsel * g.vs + g.at(0, j, i);
-  auto ld = [&](int k) { return (k >= 5 && k <= nr - 6) ? L[(long long)k * g.plane] : T(0); };
-  T q[11];
-#pragma unroll
-  for (int d = 0; d < 11; ++d) q[d] = ld(d - 5);     // planes m-5 .. m+5 for m = 0
-  for (int m = 0; m < nr; ++m) {
-    T s = Coef<T>::filtr(0) * q[5];
-#pragma unroll
-    for (int d = 1; d <= 5; ++d) s += Coef<T>::filtr(d) * (q[5 - d] + q[5 + d]);
-    U[(long long)m * g.plane] = s;
-#pragma unroll
-    for (int d = 0; d < 10; ++d) q[d] = q[d + 1];
-    q[10] = ld(m + 6);
+  const int tiles_x = n / TX, tiles = tiles_x * (n / TY);
+  int unit = blockIdx.x, ko0 = 0, ko1 = nr;
+  if (unit >= a.whole) {
+    const int t = unit - a.whole, c = t % a.chunks;
+    unit = a.whole + t / a.chunks;
+    ko0 = c * nr / a.chunks;
+    ko1 = (c + 1) * nr / a.chunks;
   }
-}
-
-// FILTER_XI^T (FILTER_ETA^T (u)) for one TX x TY tile of one field volume, plane by plane:
-// the transposes of the two in-face filters of FILTER_EXP with zero halos.  u (the adjoint
-// of the eta filter's output) lives on the face interior only.  Each thread owns V consecutive points
-// (V = 16 bytes / sizeof(T)) of one tile row.  Per plane: the box of u (tile rows +-3, tile
-// columns -4 .. +3, zero outside the face) goes to shared memory; every thread eta-filters
-// its row over the box's vector columns (the first two thread columns also take the two
-// halo vectors); threads next to an S/N face edge write the eta filter's halo adjoints
-// (v on the ghost rows, the unfiltered-halo part) to the frame; after a barrier each thread
-// xi-filters its V points from NV vectors of v, and the threads at a W/E face edge write
-// the xi filter's halo adjoints to the ghost columns.  u and v are double-buffered, so a
-// plane costs two barriers.  (A scalar form with one point per thread and three barriers per
-// plane took 136 us in float and 214 us in double per launch at 6 x 96^3; the reverse sweep
-// of 200 steps 252 -> 239 ms in float, 435 -> 427 ms in double.)
-template <typename T, int TX, int TY>
-__global__ void __launch_bounds__((TX / Vec16<T>::V) * TY) adj_filter_xyv_kernel(const T* __restrict__ in, T* out,
-                                                                                Geom g, int kp) {
-  constexpr int V = Vec16<T>::V, NT = TX / V, NTH = NT * TY;
-  constexpr int BW = TX + 8, BH = TY + 6, NG = BW / V;       // box: columns i0-4 .. i0+TX+3
-  constexpr int NBV = BH * NG, PER = (NBV + NTH - 1) / NTH;
-  constexpr int NV = (V + 8) / V;                            // vectors covering columns c-4 .. c+V+3
-  constexpr int Q0 = 4 / V;                                  // box vector of tile column 0
-  __shared__ __align__(16) T su[2][BH][BW];
-  __shared__ __align__(16) T sv[2][TY][BW];
-  const int n = g.n, tiles_x = n / TX;
-  const int i0 = (blockIdx.x % tiles_x) * TX, j0 = (blockIdx.x / tiles_x) * TY;
-  const int k0 = blockIdx.y * kp, k1 = min(g.nr, k0 + kp);
-  const long long vbase = (long long)blockIdx.z * g.vs;
+  const int ks = ko0 - 5, ke = ko1 + 5;                        // input planes, zero outside [5, nr-6]
+  const int tile = unit % tiles, rest = unit / tiles;
+  const int i0 = (tile % tiles_x) * TX, j0 = (tile / tiles_x) * TY;
+  const int s = rest % g.nf, face = rest / g.nf;
   const int cx = threadIdx.x, ty = threadIdx.y, tid = ty * NT + cx;
-  const T f0 = Coef<T>::filt(0), f1 = Coef<T>::filt(1), f2 = Coef<T>::filt(2), f3 = Coef<T>::filt(3);
-  int boff[PER];
-#pragma unroll
-  for (int e = 0; e < PER; ++e) {
-    const int q = tid + e * NTH;
-    const int br = q / NG, bq = q % NG;
-    const int gj = j0 - 3 + br, gi = i0 - 4 + V * bq;
-    boff[e] = (q < NBV && gj >= 0 && gj < n && gi >= 0 && gi < n) ? (JOFF + gj) * g.pitch + IOFF + gi : -1;
-  }
-  T nxt[PER][V];
-  auto fetch = [&](int k) {
-    const T* u = in + vbase + (long long)k * g.plane;
-#pragma unroll
-    for (int e = 0; e < PER; ++e) {
-      if (boff[e] >= 0) {
-        ldv(u + boff[e], nxt[e]);
-      } else {
-#pragma unroll
-        for (int c = 0; c < V; ++c) nxt[e][c] = T(0);
-      }
-    }
+  const int rb = R * ty;                     // first own row of the tile
+  const int z0 = (face * g.nf + s) * nr;
+  auto issue = [&](int k, int slot) {
+    uint64_t* b = &bars[slot];
+    mbar_expect_tx(b, L::PB * sizeof(T));
+    const bool in = k >= 5 && k < nr - 5;              // else a box beside the face, all zeros
+    tma_load_3d(smem + slot * L::P_BYTES, &a.mP, in ? i0 - 4 : n, j0 - 3, z0 + (in ? k : 5), b);
   };
-  if (k0 < k1) fetch(k0);
-  for (int k = k0; k < k1; ++k) {
-    const int b = k & 1;
-#pragma unroll
-    for (int e = 0; e < PER; ++e) {
-      const int q = tid + e * NTH;
-      if (q < NBV) stv(&su[b][q / NG][(q % NG) * V], nxt[e]);
-    }
-    __syncthreads();
-    if (k + 1 < k1) fetch(k + 1);
-    // eta^T on the tile rows, every vector column of the box
-    for (int q = cx; q < NG; q += NT) {
-      T c[7][V];
-#pragma unroll
-      for (int m = 0; m < 7; ++m) ldv(&su[b][ty + m][q * V], c[m]);
-      T v[V];
-#pragma unroll
-      for (int e = 0; e < V; ++e)
-        v[e] = f0 * c[3][e] + f1 * (c[2][e] + c[4][e]) + f2 * (c[1][e] + c[5][e]) + f3 * (c[0][e] + c[6][e]);
-      stv(&sv[b][ty][q * V], v);
-    }
-    T* o = out + vbase + (long long)k * g.plane;
-    // eta-filter halo adjoints: v on the ghost rows (box rows 0..2 / TY+3..TY+5), tile columns
-    for (int side = 0; side < 2; ++side) {
-      const bool edge = side == 0 ? (j0 == 0 && ty < 3) : (j0 + TY == n && ty >= TY - 3);
-      if (!edge) continue;
-      const int r = side == 0 ? ty : ty + 6;                 // box row
-      T v[V];
-#pragma unroll
-      for (int e = 0; e < V; ++e) v[e] = T(0);
-      auto U = [&](int br, int e) { return (br >= 0 && br < BH) ? su[b][br][(Q0 + cx) * V + e] : T(0); };
-#pragma unroll
-      for (int e = 0; e < V; ++e)
-        v[e] = f0 * U(r, e) + f1 * (U(r - 1, e) + U(r + 1, e)) + f2 * (U(r - 2, e) + U(r + 2, e)) +
-               f3 * (U(r - 3, e) + U(r + 3, e));
-      stv(o + (JOFF + j0 - 3 + r) * g.pitch + IOFF + i0 + V * cx, v);
-    }
-    __syncthreads();
-    // xi^T on the tile: w holds box columns V*cx .. V*cx + NV*V - 1; the own point e sits at
-    // box column V*cx + 4 + e
+  if (tid == 0) {
+    for (int q = 0; q < kFiltRing; ++q) mbar_init(&bars[q], 1);
+    mbar_fence_init();
+  }
+  __syncthreads();
+  // No wait here: adj_ghost_kernel, launched before this one, releases it only after its own wait,
+  // so the kernels before that one are complete; the two run side by side (this one waits at
+  // its end).
+  const bool loads = !a.wc.no_loads;
+  if (tid == 0 && loads)
+    for (int k = ks; k < min(ks + kFiltRing, ke); ++k) issue(k, k - ks);
+  T* out = a.qout + g.vol(0, face, s) + g.at(0, j0 + rb, i0 + V * cx);
+  constexpr T f0 = T(kFilt[0]), f1 = T(kFilt[1]), f2 = T(kFilt[2]), f3 = T(kFilt[3]);
+  constexpr T rw[6] = {T(kFiltR[0]), T(kFiltR[1]), T(kFiltR[2]), T(kFiltR[3]), T(kFiltR[4]), T(kFiltR[5])};
+  auto xi_row = [&](const T* bx, int r, T* v) {       // xi filter of box row r at the own columns
     T w[NV * V];
 #pragma unroll
-    for (int m = 0; m < NV; ++m) ldv(&sv[b][ty][(cx + m) * V], w + m * V);
-    auto W = [&](int idx) { return (idx >= 0 && idx < NV * V) ? w[idx] : T(0); };
-    auto xt = [&](int c) {                                   // c = index into w
-      return f0 * W(c) + f1 * (W(c - 1) + W(c + 1)) + f2 * (W(c - 2) + W(c + 2)) + f3 * (W(c - 3) + W(c + 3));
-    };
-    T r[V];
+    for (int m = 0; m < NV; ++m) ldv(bx + r * PW + V * cx + m * V, w + m * V);
 #pragma unroll
-    for (int e = 0; e < V; ++e) r[e] = xt(4 + e);
-    stv(o + (JOFF + j0 + ty) * g.pitch + IOFF + i0 + V * cx, r);
-    // xi-filter halo adjoints on the ghost columns (box columns 1..3 / TX+4..TX+6)
-    if (i0 == 0 && cx == 0) {
+    for (int q = 0; q < V; ++q)
+      v[q] = f0 * w[4 + q] + f1 * (w[3 + q] + w[5 + q]) + f2 * (w[2 + q] + w[6 + q]) + f3 * (w[1 + q] + w[7 + q]);
+  };
+  // radial queue of eta-filtered planes, in float as packed pairs (filter_kernel)
+  T tq[11][R][V];
+  unsigned long long tq2[11][R][NP];
 #pragma unroll
-      for (int c = 1; c <= 3; ++c) o[(JOFF + j0 + ty) * g.pitch + IOFF - 4 + c] = xt(c);
+  for (int m = 0; m < 11; ++m)
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+      for (int q = 0; q < V; ++q) tq[m][r][q] = T(0);
+#pragma unroll
+      for (int h = 0; h < NP; ++h) tq2[m][r][h] = 0ull;
     }
-    if (i0 + TX == n && cx == NT - 1) {
+  // A thread whose wait gives up reports it at the CTA barrier; the CTA leaves the plane loop
+  // there (fail_at = 2 * plane + whether thread 0's own wait on that plane succeeded).
+  bool ok = true;
+  int fail_at = 0;
+  int slot = 0;
+  uint32_t phase = 0;
+  for (int kb = ks; kb < ke && ok; kb += 11) {
 #pragma unroll
-      for (int c = TX + 4; c <= TX + 6; ++c) o[(JOFF + j0 + ty) * g.pitch + IOFF + i0 - 4 + c] = xt(c - V * cx);
+    for (int u = 0; u < 11; ++u) {
+      const int k = kb + u;
+      if (k >= ke) break;
+      {
+        const bool got = mbar_wait(&bars[slot], phase, a.wc, kErrAdjointRing);
+        const T* bx = reinterpret_cast<const T*>(smem + slot * L::P_BYTES);
+        T* t1 = reinterpret_cast<T*>(smem + kFiltRing * L::P_BYTES + (k & 1) * L::S_BYTES);
+        T c[R + 6][V];                                 // c[m] holds xi-filtered box row rb + m
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          xi_row(bx, rb + 3 + r, c[3 + r]);
+          stv(t1 + (rb + 3 + r) * TX + V * cx, c[3 + r]);
+        }
+        for (int h = ty; h < 6; h += NY) {             // the halo rows of the box
+          const int r = h < 3 ? h : TY + h;
+          T v[V];
+          xi_row(bx, r, v);
+          stv(t1 + r * TX + V * cx, v);
+        }
+        if (__syncthreads_or(!got)) { ok = false; fail_at = 2 * k + (got ? 1 : 0); break; }
+        if (tid == 0 && loads && k + kFiltRing < ke) issue(k + kFiltRing, slot);
+        if (++slot == kFiltRing) { slot = 0; phase ^= 1; }
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+          ldv(t1 + (rb + m) * TX + V * cx, c[m]);
+          ldv(t1 + (rb + R + 3 + m) * TX + V * cx, c[R + 3 + m]);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          if constexpr (PAIRS) {
+#pragma unroll
+            for (int h = 0; h < NP; ++h) {
+              auto pr = [&](int m) { return pk2(c[r + m][2 * h], c[r + m][2 * h + 1]); };
+              unsigned long long t = mul2(pk2(f0, f0), pr(3));
+              t = fma2(pk2(f1, f1), add2(pr(2), pr(4)), t);
+              t = fma2(pk2(f2, f2), add2(pr(1), pr(5)), t);
+              tq2[u][r][h] = fma2(pk2(f3, f3), add2(pr(0), pr(6)), t);
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < V; ++q)
+              tq[u][r][q] = f0 * c[r + 3][q] + f1 * (c[r + 2][q] + c[r + 4][q]) + f2 * (c[r + 1][q] + c[r + 5][q]) +
+                            f3 * (c[r][q] + c[r + 6][q]);
+          }
+        }
+      }
+      if (k >= ko0 + 5) {
+        // planes k-10 .. k sit at queue rows (u+1 .. u+11) % 11; the centre is k-5
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          T v[V];
+          if constexpr (PAIRS) {
+#pragma unroll
+            for (int h = 0; h < NP; ++h) {
+              unsigned long long acc = mul2(pk2(rw[0], rw[0]), tq2[(u + 6) % 11][r][h]);
+#pragma unroll
+              for (int m = 1; m <= 5; ++m)
+                acc = fma2(pk2(rw[m], rw[m]), add2(tq2[(u + 6 - m) % 11][r][h], tq2[(u + 6 + m) % 11][r][h]), acc);
+              float x, y;
+              upk2(acc, x, y);
+              v[2 * h] = x;
+              v[2 * h + 1] = y;
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < V; ++q) {
+              T acc = rw[0] * tq[(u + 6) % 11][r][q];
+#pragma unroll
+              for (int m = 1; m <= 5; ++m) acc += rw[m] * (tq[(u + 6 - m) % 11][r][q] + tq[(u + 6 + m) % 11][r][q]);
+              v[q] = acc;
+            }
+          }
+          stv(out + (long long)(k - 5) * g.plane + r * g.pitch, v);
+        }
+      }
     }
+  }
+  if (!ok && tid == 0 && loads) {
+    // at the break on plane k, planes [ks, min(k + kFiltRing, ke)) were issued
+    const int k = fail_at >> 1;
+    mbar_drain(bars, kFiltRing, ks, k + (fail_at & 1), min(k + kFiltRing, ke), a.wc.polls);
+  }
+  grid_dependency_wait();
+}
+
+// Ghost adjoints of FILTER_EXP^T, from the interior of `in` into the frame of `out`.  The eta
+// filter's halo took the unfiltered rows, so the ghost rows are the eta transpose of u alone,
+// sums of the three rows next to the edge; the ghost columns are the xi transpose of eta^T u,
+// sums of the three columns next to it.  Both are then filtered radially, with an 11-deep
+// register queue of the three values per thread, over a chunk of kp planes.  grid.z: volume and
+// edge.  Ghost rows: one thread per column.  Ghost columns: one lane per row, which reads the
+// aligned group of four values once per plane and takes its neighbours' from the other lanes
+// (lanes 3..28 write); reading 7 rows per thread, or one layer per thread, is bound by the
+// scattered requests.
+template <typename T>
+struct AdjGhostArgs {
+  const T* in;
+  T* out;
+  Geom g;
+  int kp;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(128) adj_ghost_kernel(const __grid_constant__ AdjGhostArgs<T> a) {
+  const Geom& g = a.g;
+  const int n = g.n, nr = g.nr;
+  const int e = blockIdx.z & 3;
+  const T* in = a.in + (long long)(blockIdx.z >> 2) * g.vs;
+  T* out = a.out + (long long)(blockIdx.z >> 2) * g.vs;
+  const int k0 = blockIdx.y * a.kp, k1 = min(nr, k0 + a.kp);
+  constexpr T f0 = T(kFilt[0]), f1 = T(kFilt[1]), f2 = T(kFilt[2]), f3 = T(kFilt[3]);
+  constexpr T rw[6] = {T(kFiltR[0]), T(kFiltR[1]), T(kFiltR[2]), T(kFiltR[3]), T(kFiltR[4]), T(kFiltR[5])};
+  const bool cols = e >= 2;
+  const int lane = threadIdx.x & 31, gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int t = cols ? gw * 26 + lane - 3 : (int)(blockIdx.x * blockDim.x + threadIdx.x);   // row or column
+  const bool in_face = t >= 0 && t < n, writes = in_face && (!cols || (lane >= 3 && lane < 29));
+  grid_dependency_wait();
+  release_dependents();                                      // after the wait: adj_filter_kernel relies on it
+  if (cols ? gw * 26 >= n : t >= n) return;                  // whole warps (columns) or lone threads
+  // the three values next to the edge of plane k, nearest first (eta-filtered for the columns)
+  auto load = [&](int k, T* v) {
+    v[0] = v[1] = v[2] = T(0);
+    if (k < 5 || k > nr - 6) return;                         // uniform over the grid's block row
+    if (!cols) {
+#pragma unroll
+      for (int l = 0; l < 3; ++l) v[l] = in[g.at(k, e == 0 ? l : n - 1 - l, t)];
+      return;
+    }
+    T u[4] = {T(0), T(0), T(0), T(0)};
+    if (in_face) {
+      const T* p = in + g.at(k, t, e == 2 ? 0 : n - 4);
+      ldv(p, u);
+      if (sizeof(T) == 8) ldv(p + 2, u + 2);
+    }
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+      const T x = e == 2 ? u[l] : u[3 - l];
+      T s = f0 * x;
+      s += f1 * (__shfl_up_sync(0xffffffffu, x, 1) + __shfl_down_sync(0xffffffffu, x, 1));
+      s += f2 * (__shfl_up_sync(0xffffffffu, x, 2) + __shfl_down_sync(0xffffffffu, x, 2));
+      s += f3 * (__shfl_up_sync(0xffffffffu, x, 3) + __shfl_down_sync(0xffffffffu, x, 3));
+      v[l] = s;
+    }
+  };
+  T q[11][3];
+#pragma unroll
+  for (int d = 0; d < 11; ++d) load(k0 + d - 5, q[d]);       // planes m-5 .. m+5 for m = k0
+  for (int m = k0; m < k1; ++m) {
+    T s[3];
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+      s[l] = rw[0] * q[5][l];
+#pragma unroll
+      for (int d = 1; d <= 5; ++d) s[l] += rw[d] * (q[5 - d][l] + q[5 + d][l]);
+    }
+    const T w[3] = {f1 * s[0] + f2 * s[1] + f3 * s[2], f2 * s[0] + f3 * s[1], f3 * s[0]};   // layers 1, 2, 3
+    if (writes) {
+      if (!cols) {
+#pragma unroll
+        for (int l = 0; l < 3; ++l) out[g.at(m, e == 0 ? -1 - l : n + l, t)] = w[l];
+      } else {                                               // the group of four: columns -4..-1 or n..n+3
+        T v[4];
+#pragma unroll
+        for (int l = 0; l < 3; ++l) v[e == 2 ? 3 - l : l] = w[l];
+        v[e == 2 ? 0 : 3] = T(0);
+        T* p = out + g.at(m, t, e == 2 ? -4 : n);
+        stv(p, v);
+        if (sizeof(T) == 8) stv(p + 2, v + 2);
+      }
+    }
+#pragma unroll
+    for (int d = 0; d < 10; ++d)
+#pragma unroll
+      for (int l = 0; l < 3; ++l) q[d][l] = q[d + 1][l];
+    load(m + 6, q[10]);
   }
 }
 

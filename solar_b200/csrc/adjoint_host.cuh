@@ -148,26 +148,47 @@ static int enqueue_rhs_adjoint(solar_ctx* c, AdjStageArgs<T> a, bool last) {
   return SOLAR_OK;
 }
 
-// FILTER_EXP^T in place on buffer L: radial^T, eta^T, xi^T, then the halo scatter.
+template <typename T, int TX, int TY, int R>
+static int launch_adj_filter(solar_ctx* c) {
+  using L = FilterLayout<T, TX, TY>;
+  AdjBuffers& b = c->adj;
+  const Geom& g = c->g;
+  FilterArgs<T> a;
+  if (!make_interior_map(c, b.L, TX + 8, TY + 6, &a.mP)) return fail(SOLAR_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+  a.qout = (T*)b.T1;
+  a.runs = nullptr;
+  a.wc = wait_ctl(c, kInjAdjStage);
+  a.g = g;
+  constexpr int threads = (TX / Vec16<T>::V) * (TY / R);
+  static bool attr_set = false;
+  static int resident = 1;
+  if (!attr_set) {
+    CK(cudaFuncSetAttribute(adj_filter_kernel<T, TX, TY, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::TOTAL));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, adj_filter_kernel<T, TX, TY, R>, threads, L::TOTAL));
+    resident = std::max(resident, 1);
+    attr_set = true;
+  }
+  const long long units = (long long)(g.n / TX) * (g.n / TY) * g.nf * 6;
+  const long long grid = split_units(units, g.nr, c->nsm, resident, &a.whole, &a.chunks);
+  CK(launch_pdl(adj_filter_kernel<T, TX, TY, R>, dim3((unsigned)grid), dim3(TX / Vec16<T>::V, TY / R), L::TOTAL, c->stream, a));
+  return SOLAR_OK;
+}
+
+// FILTER_EXP^T on buffer L (which takes the scratch buffer's place and the other way round).
 template <typename T>
 static int enqueue_filter_adjoint(solar_ctx* c) {
   const Geom& g = c->g;
-  T* L = (T*)c->adj.L;
-  T* T1 = (T*)c->adj.T1;
-  adj_filter_r_kernel<T><<<blocks_for(6LL * g.nf * g.n * g.n, 128), 128, 0, c->stream>>>(L, T1, g);
-  constexpr int KP = 8;                                             // planes per CTA
-  const unsigned kch = (unsigned)((g.nr + KP - 1) / KP);
-  constexpr int V = Vec16<T>::V;
-  if (g.n % 32 == 0) {
-    constexpr int TY = sizeof(T) == 4 ? 16 : 8;
-    adj_filter_xyv_kernel<T, 32, TY><<<dim3((g.n / 32) * (g.n / TY), kch, 6 * g.nf), dim3(32 / V, TY), 0, c->stream>>>(
-        T1, L, g, KP);
-  } else {
-    adj_filter_xyv_kernel<T, 16, 16><<<dim3((g.n / 16) * (g.n / 16), kch, 6 * g.nf), dim3(16 / V, 16), 0, c->stream>>>(
-        T1, L, g, KP);
-  }
+  AdjBuffers& b = c->adj;
+  AdjGhostArgs<T> a = {(const T*)b.L, (T*)b.T1, g, 16};             // 16 planes per thread
+  const int warps = std::max((g.n + 31) / 32, (g.n + 25) / 26);     // a column warp writes 26 rows
+  CK(launch_pdl(adj_ghost_kernel<T>, dim3((unsigned)(warps + 3) / 4, (unsigned)((g.nr + a.kp - 1) / a.kp), 24 * g.nf), dim3(128),
+                0, c->stream, a));
+  constexpr int R = sizeof(T) == 4 ? 1 : 2;                         // as launch_filter
+  int rc = g.n % 32 == 0 ? launch_adj_filter<T, 32, 16, R>(c) : launch_adj_filter<T, 16, 16, R>(c);
+  if (rc) return rc;
+  std::swap(b.L, b.T1);
   adj_edge_kernel<T><<<dim3(blocks_for(g.n, 128), 72, g.nr), 128, g.nf * g.n * sizeof(T), c->stream>>>(
-      L, nullptr, T(0), (const T*)c->adj.wt, c->adj.wt_span, c->adj.tspan, g, 1);
+      (T*)b.L, nullptr, T(0), (const T*)b.wt, b.wt_span, b.tspan, g, 1);
   CK(cudaGetLastError());
   return SOLAR_OK;
 }

@@ -339,6 +339,23 @@ static bool make_map(const solar_ctx* c, const void* base, int bx, int by, CUten
   return r == CUDA_SUCCESS;
 }
 
+// 3-D view of the face interiors of a buffer: x = i, y = j, z as above; boxes are filled with
+// zeros outside the face.
+static bool make_interior_map(const solar_ctx* c, const void* base, int bx, int by, CUtensorMap* m) {
+  auto enc = tensor_map_encoder();
+  if (!enc) return false;
+  const Geom& g = c->g;
+  cuuint64_t dims[3] = {(cuuint64_t)g.n, (cuuint64_t)g.n, (cuuint64_t)g.nruns * 6 * g.nf * g.nr};
+  cuuint64_t strides[2] = {(cuuint64_t)g.pitch * c->esize, (cuuint64_t)g.plane * c->esize};
+  cuuint32_t box[3] = {(cuuint32_t)bx, (cuuint32_t)by, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  void* first = (char*)const_cast<void*>(base) + (size_t)g.at(0, 0, 0) * c->esize;   // on a 32-byte boundary
+  CUresult r = enc(m, c->fp32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, first, dims,
+                   strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS;
+}
+
 // 4-D view of a whole buffer: x, y as above, z = k, w = volume ((run*6 + face)*nf + slot); box
 // bx x by x 1 x nfields, the boxes of consecutive slots one after the other.
 static bool make_fields_map(const solar_ctx* c, const void* base, int bx, int by, int nfields, CUtensorMap* m) {
@@ -597,6 +614,41 @@ static int launch_stage(solar_ctx* c, const void* qin, void* qout, int mode, int
   return fail(SOLAR_ERR_ARG, "unsupported stage tile %d x %d", tx, ty);
 }
 
+// Work split of the filter kernels: `units` (tile, field, volume) columns of nk planes; returns
+// the CTAs launched.
+static long long split_units(long long units, long long nk, int nsm, int resident, int* whole, int* chunks_out) {
+  // Whole-column CTAs for every full wave; the units of a last, partial wave are cut into
+  // radial chunks (at least 11 planes each) so that they fill one wave.  When every unit
+  // fits in one wave, SMs would hold units / nsm or one more whole column: the units past
+  // an even share are cut into chunks, about one per SM, which run in the spare CTA slot
+  // beside the whole columns (6 x 128^3 float: 740 columns and 140 chunks of 118 / 5
+  // planes instead of 28 SMs with six columns).
+  const long long slots = (long long)nsm * resident;
+  *whole = (int)units;
+  *chunks_out = 1;
+  long long cut = 0, chunks = 1;
+  if (units > slots) {
+    cut = units % slots;
+    if (cut > 0) chunks = std::min<long long>(nk / 11, std::max<long long>(1, (slots + cut / 2) / cut));
+  } else if (2 * units <= slots && nk >= 22) {
+    // Two or more chunks of every unit fit in one wave: the march through the planes is the
+    // kernel's time, so every unit is cut (us per step at 6 x 64^3, float: 3 chunks 175, whole
+    // columns and 44 cut ones 185; 6 x 32^3: 2 chunks 69.7 in float, 93.5 in double, whole 73.8,
+    // 98.4; chunks shorter than 11 planes gain nothing, they re-read 10).
+    cut = units;
+    chunks = std::min<long long>(nk / 11, slots / units);
+  } else {
+    const long long per = units / nsm;
+    cut = units % nsm;
+    if (per >= 1 && per < resident && cut > 0) chunks = std::min<long long>(nk / 11, nsm / cut);
+  }
+  if (chunks > 1) {
+    *whole = (int)(units - cut);
+    *chunks_out = (int)chunks;
+  }
+  return *whole + (units - *whole) * *chunks_out;
+}
+
 template <typename T, int TX, int TY, int R>
 static int launch_filter_t(solar_ctx* c, const void* qin, void* qout, const int* runs) {
   using L = FilterLayout<T, TX, TY>;
@@ -615,38 +667,8 @@ static int launch_filter_t(solar_ctx* c, const void* qin, void* qout, const int*
     resident = std::max(resident, 1);
     attr_set = true;
   }
-  // Whole-column CTAs for every full wave; the units of a last, partial wave are cut into
-  // radial chunks (at least 11 planes each) so that they fill one wave.  When every unit
-  // fits in one wave, SMs would hold units / nsm or one more whole column: the units past
-  // an even share are cut into chunks, about one per SM, which run in the spare CTA slot
-  // beside the whole columns (6 x 128^3 float: 740 columns and 140 chunks of 118 / 5
-  // planes instead of 28 SMs with six columns).
   const long long units = (long long)(c->g.n / TX) * (c->g.n / TY) * c->g.nf * launched_runs(c, runs) * c->g.nface;
-  const long long slots = (long long)c->nsm * resident;
-  const long long nk = c->g.k1 - c->g.k0;
-  a.whole = (int)units;
-  a.chunks = 1;
-  long long cut = 0, chunks = 1;
-  if (units > slots) {
-    cut = units % slots;
-    if (cut > 0) chunks = std::min<long long>(nk / 11, std::max<long long>(1, (slots + cut / 2) / cut));
-  } else if (2 * units <= slots && nk >= 22) {
-    // Two or more chunks of every unit fit in one wave: the march through the planes is the
-    // kernel's time, so every unit is cut (us per step at 6 x 64^3, float: 3 chunks 175, whole
-    // columns and 44 cut ones 185; 6 x 32^3: 2 chunks 69.7 in float, 93.5 in double, whole 73.8,
-    // 98.4; chunks shorter than 11 planes gain nothing, they re-read 10).
-    cut = units;
-    chunks = std::min<long long>(nk / 11, slots / units);
-  } else {
-    const long long per = units / c->nsm;
-    cut = units % c->nsm;
-    if (per >= 1 && per < resident && cut > 0) chunks = std::min<long long>(nk / 11, c->nsm / cut);
-  }
-  if (chunks > 1) {
-    a.whole = (int)(units - cut);
-    a.chunks = (int)chunks;
-  }
-  const long long grid = a.whole + (units - a.whole) * a.chunks;
+  const long long grid = split_units(units, c->g.k1 - c->g.k0, c->nsm, resident, &a.whole, &a.chunks);
   CK(launch_pdl(filter_kernel<T, TX, TY, R>, dim3((unsigned)grid), dim3(TX / Vec16<T>::V, TY / R), L::TOTAL, c->stream, a));
   return SOLAR_OK;
 }
