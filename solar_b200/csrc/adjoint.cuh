@@ -247,6 +247,7 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
   const int to = ty * TX + V * cx;                 // own points in a tile
   const T k2 = -a.dt * a.inv_dxi;
   for (int m = kb - 3; m <= ke + 2; ++m) {
+    if (m == ke + 1) release_dependents();
     const bool real = (m >= 0 && m < nr);
     const bool own = (m >= kb && m < ke);
     const bool bc = (m == 0 || m == nr - 1);
@@ -542,8 +543,26 @@ __global__ void grad_scale_kernel(double* grad, const T* c2, const T* radT, int 
 // field scalar.  grid: x over u, y over (receiving face-edge, layer), z over planes; dynamic
 // shared memory: (mode 0 ? 2 : nf) x n values.
 template <typename T>
-__global__ void adj_edge_kernel(T* q, T* mu, T beta, const T* __restrict__ wt, int span, const int* __restrict__ tspan,
-                                Geom g, int mode) {
+struct AdjEdgeArgs {
+  T* q;
+  T* mu;                  // or nullptr
+  T beta;
+  const T* wt;
+  int span;
+  const int* tspan;
+  Geom g;
+  int mode;
+};
+
+template <typename T>
+__global__ void adj_edge_kernel(const __grid_constant__ AdjEdgeArgs<T> a) {
+  T* const q = a.q;
+  T* const mu = a.mu;
+  const T beta = a.beta;
+  const T* __restrict__ wt = a.wt;
+  const int* __restrict__ tspan = a.tspan;
+  const int span = a.span, mode = a.mode;
+  const Geom& g = a.g;
   extern __shared__ __align__(16) unsigned char aesm[];
   T* const sg = reinterpret_cast<T*>(aesm);               // [field][t]
   __shared__ int s_lo, s_hi;
@@ -565,6 +584,8 @@ __global__ void adj_edge_kernel(T* q, T* mu, T beta, const T* __restrict__ wt, i
   if (hi >= lo) { atomicMin(&s_lo, lo); atomicMax(&s_hi, hi); }
   __syncthreads();
   const int tmin = s_lo, tmax = s_hi;
+  grid_dependency_wait();                                  // constant tables only above
+  release_dependents();
   if (tmax < tmin) return;                                 // no ghost point uses this block
   // receiver ghost position of (e, l, t): rows -1-l / n+l, columns -1-l / n+l
   const long long g0 = (e == 0) ? g.at(k, -1 - l, 0) : (e == 1) ? g.at(k, n + l, 0)

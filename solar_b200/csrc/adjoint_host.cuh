@@ -140,9 +140,8 @@ static int enqueue_rhs_adjoint(solar_ctx* c, AdjStageArgs<T> a, bool last) {
     return fail(SOLAR_ERR_ARG, "grid too large for the adjoint (%lld values per face)", (long long)g.nf * g.vs);
   int rc = (g.n % 32 == 0) ? launch_adj_stage<T, 32, 8>(c, a) : launch_adj_stage<T, 16, 16>(c, a);
   if (rc) return rc;
-  adj_edge_kernel<T><<<dim3(blocks_for(g.n, 128), 72, g.nr), 128, 2 * g.n * sizeof(T), c->stream>>>(
-      a.lout, a.muout, a.beta_next, (const T*)b.wt, b.wt_span, b.tspan, g, 0);
-  CK(cudaGetLastError());
+  const AdjEdgeArgs<T> ae = {a.lout, a.muout, a.beta_next, (const T*)b.wt, b.wt_span, b.tspan, g, 0};
+  CK(launch_pdl(adj_edge_kernel<T>, dim3(blocks_for(g.n, 128), 72, g.nr), dim3(128), 2 * g.n * sizeof(T), c->stream, ae));
   std::swap(b.L, b.T1);
   std::swap(b.LW, b.T2);
   return SOLAR_OK;
@@ -187,9 +186,8 @@ static int enqueue_filter_adjoint(solar_ctx* c) {
   int rc = g.n % 32 == 0 ? launch_adj_filter<T, 32, 16, R>(c) : launch_adj_filter<T, 16, 16, R>(c);
   if (rc) return rc;
   std::swap(b.L, b.T1);
-  adj_edge_kernel<T><<<dim3(blocks_for(g.n, 128), 72, g.nr), 128, g.nf * g.n * sizeof(T), c->stream>>>(
-      (T*)b.L, nullptr, T(0), (const T*)b.wt, b.wt_span, b.tspan, g, 1);
-  CK(cudaGetLastError());
+  const AdjEdgeArgs<T> ae = {(T*)b.L, nullptr, T(0), (const T*)b.wt, b.wt_span, b.tspan, g, 1};
+  CK(launch_pdl(adj_edge_kernel<T>, dim3(blocks_for(g.n, 128), 72, g.nr), dim3(128), g.nf * g.n * sizeof(T), c->stream, ae));
   return SOLAR_OK;
 }
 
