@@ -218,7 +218,7 @@ static int enqueue_step_div(solar_ctx* c, T* dstep) {
   void* bufs[2] = {c->A, c->B};
   const long long V6 = 6 * vol_compact(c);
   int cur = 0, rc;
-  if ((rc = force_begin(c))) return rc;
+  if ((rc = force_begin(c, true))) return rc;
   for (int s = 0; s < 5; ++s) {
     if ((rc = launch_edge<T>(c, bufs[cur], 0, nullptr))) return rc;
     if ((rc = launch_stage<T>(c, bufs[cur], bufs[cur ^ 1], s == 0 ? 4 : 5, s, nullptr, dstep + s * V6))) return rc;
@@ -227,7 +227,7 @@ static int enqueue_step_div(solar_ctx* c, T* dstep) {
   if ((rc = launch_edge<T>(c, bufs[cur], 1, nullptr))) return rc;
   if ((rc = launch_filter<T>(c, bufs[cur], bufs[cur ^ 1], nullptr))) return rc;
   CK(cudaGetLastError());
-  return force_end(c);
+  return SOLAR_OK;
 }
 
 template <typename T>

@@ -12,8 +12,8 @@
 // timestep.f90:82).  A one-thread clock kernel at the start of each step evaluates the
 // time factors (including the reference's coefficient refresh when floor(xt) advances),
 // a field kernel forms this step's S(x, y) for all faces, the stage kernel adds S(x, y)
-// times the radial factor to the v_r right-hand side, and a clock kernel after the filter
-// advances time and step.
+// times the radial factor to the v_r right-hand side; the field kernel advances time and step
+// for the next one.
 #pragma once
 
 namespace solar {
@@ -29,8 +29,21 @@ struct ForceClock {
   double mag;           // analytic magnitude at this step
 };
 
-__global__ void force_clock_kernel(ForceClock* c, int kind, double diml, double dimc, double dt, double cad, int nstep,
-                                   int nt, int* err) {
+struct ForceClockArgs {
+  ForceClock* c;
+  int kind;
+  double diml, dimc, dt, cad;
+  int nstep, nt;
+  int* err;
+};
+
+__global__ void force_clock_kernel(const __grid_constant__ ForceClockArgs a) {
+  ForceClock* const c = a.c;
+  const int kind = a.kind, nstep = a.nstep, nt = a.nt;
+  const double diml = a.diml, dimc = a.dimc, dt = a.dt, cad = a.cad;
+  int* const err = a.err;
+  grid_dependency_wait();
+  release_dependents();
   if (threadIdx.x || blockIdx.x) return;
   if (kind == SOLAR_FORCING_ANALYTIC) {
     const double u = c->time * diml / dimc - 650.0;
@@ -62,10 +75,35 @@ __global__ void force_clock_kernel(ForceClock* c, int kind, double diml, double 
 }
 
 template <typename T>
-__global__ void force_field_kernel(const ForceClock* c, int kind, const double* exy, const double* samples,
-                                   long long n6, T* out) {
+struct ForceFieldArgs {
+  ForceClock* c;
+  int kind;
+  const double* exy;
+  const double* samples;
+  long long n6;
+  T* out;
+  double dt;
+  int advance;              // the step's time += dt, step += 1
+};
+
+// The field does not depend on the time and step words, so one thread advances them for the
+// next step here (a kernel of its own after the filter cost 3 us a step).
+template <typename T>
+__global__ void force_field_kernel(const __grid_constant__ ForceFieldArgs<T> a) {
+  ForceClock* const c = a.c;
+  const int kind = a.kind;
+  const double* exy = a.exy;
+  const double* samples = a.samples;
+  const long long n6 = a.n6;
+  T* const out = a.out;
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  grid_dependency_wait();
+  release_dependents();
   if (p >= n6) return;
+  if (p == 0 && a.advance) {
+    c->time = c->time + a.dt;
+    c->step = c->step + 1;
+  }
   if (kind == SOLAR_FORCING_ANALYTIC) {
     out[p] = (T)(c->mag * exy[p]);
     return;
@@ -84,12 +122,6 @@ __global__ void force_field_kernel(const ForceClock* c, int kind, const double* 
   out[p] = (T)f;
 }
 
-__global__ void force_advance_kernel(ForceClock* c, double dt) {
-  if (threadIdx.x || blockIdx.x) return;
-  c->time = c->time + dt;
-  c->step = c->step + 1;
-}
-
 // Nearest plane to r (ties to the outer plane), as SOLAR_DATA picks e_rad and o_rad.
 static int nearest_plane(const solar_ctx* c, double r) {
   double temp = 1.0;
@@ -102,27 +134,23 @@ static int nearest_plane(const solar_ctx* c, double r) {
   return o;
 }
 
-static int force_begin(solar_ctx* c) {
-  if (!c->forcing) return SOLAR_OK;
-  force_clock_kernel<<<1, 1, 0, c->stream>>>((ForceClock*)c->force_clock, c->forcing, 695.9894e8, c->ht.dimc,
-                                             c->desc.dt, c->force_cad, c->force_nstep, c->force_nt, c->err);
+template <typename T>
+static int launch_force_field(solar_ctx* c, bool advance) {
   const long long n6 = 6LL * c->g.n * c->g.n;
-  const unsigned blocks = (unsigned)((n6 + 255) / 256);
-  if (c->fp32)
-    force_field_kernel<float><<<blocks, 256, 0, c->stream>>>((const ForceClock*)c->force_clock, c->forcing,
-                                                             c->force_exy, c->force_samples, n6, (float*)c->force_xy);
-  else
-    force_field_kernel<double><<<blocks, 256, 0, c->stream>>>((const ForceClock*)c->force_clock, c->forcing,
-                                                              c->force_exy, c->force_samples, n6, (double*)c->force_xy);
-  CK(cudaGetLastError());
+  const ForceFieldArgs<T> a = {(ForceClock*)c->force_clock, c->forcing, c->force_exy, c->force_samples, n6, (T*)c->force_xy,
+                               c->desc.dt, advance ? 1 : 0};
+  CK(launch_pdl(force_field_kernel<T>, dim3((unsigned)((n6 + 255) / 256)), dim3(256), 0, c->stream, a));
   return SOLAR_OK;
 }
 
-static int force_end(solar_ctx* c) {
+// The source field of the current step; `advance`: the step is taken (the operators leave the
+// clock as it is).
+static int force_begin(solar_ctx* c, bool advance) {
   if (!c->forcing) return SOLAR_OK;
-  force_advance_kernel<<<1, 1, 0, c->stream>>>((ForceClock*)c->force_clock, c->desc.dt);
-  CK(cudaGetLastError());
-  return SOLAR_OK;
+  const ForceClockArgs a = {(ForceClock*)c->force_clock, c->forcing, 695.9894e8, c->ht.dimc, c->desc.dt, c->force_cad,
+                            c->force_nstep, c->force_nt, c->err};
+  CK(launch_pdl(force_clock_kernel, dim3(1), dim3(1), 0, c->stream, a));
+  return c->fp32 ? launch_force_field<float>(c, advance) : launch_force_field<double>(c, advance);
 }
 
 template <typename T>
@@ -196,7 +224,7 @@ int solar_gpu_set_forcing(solar_ctx* c, int kind, int k_center, int nstep) {
     if (rc) return rc;
   }
   c->forcing = kind;
-  if (c->step_graph) { cudaGraphExecDestroy(c->step_graph); c->step_graph = nullptr; }
+  drop_step_graphs(c);
   drop_batch_graphs(c);
   return SOLAR_OK;
 }

@@ -192,10 +192,13 @@ struct solar_ctx {
   long long steps_done = 0;    // steps taken by this context (watchdog step numbers)
   double* norm_ring = nullptr; // per-step sums of squares (solar_gpu_rk4_norms)
   int norm_ring_len = 0;
+  int* norm_ctl = nullptr;     // SumsqArgs::ctl
   DevTables dt;
   int tile_x = 32, tile_y = 8, kchunk = 0;
   int edge_resident = 0;       // edge-kernel CTAs per SM (threads and shared memory depend on nx)
   cudaGraphExec_t step_graph = nullptr;
+  cudaGraphExec_t norm_graph = nullptr;   // a step and the sum of squares of one field ...
+  int norm_run = 0, norm_slot = 0;        // ... of this run and slot, into norm_ring
   std::vector<cudaGraphExec_t> batch_graphs;   // batched step graph per number of live runs
   cudaEvent_t ev[8] = {};
   // FP32 contexts upload the state across PCIe as float: two pinned blocks of one compact
@@ -684,8 +687,7 @@ static int launch_filter(solar_ctx* c, const void* qin, void* qout, const int* r
   return launch_filter_t<T, 16, 16, R>(c, qin, qout, runs);
 }
 
-static int force_begin(solar_ctx* c);   // forcing.cuh: this step's source field
-static int force_end(solar_ctx* c);     // forcing.cuh: time += dt, step += 1
+static int force_begin(solar_ctx* c, bool advance);   // forcing.cuh: this step's source field, its clock
 
 // One full time step (timestep.f90:61-82) on every run.  With ev != nullptr each kernel
 // is bracketed by events: ev_pairs[kind] accumulates into times[kind].
@@ -693,7 +695,7 @@ template <typename T>
 static int enqueue_step(solar_ctx* c, const int* runs, std::vector<cudaEvent_t>* evs) {
   void* bufs[2] = {c->A, c->B};
   int cur = 0, rc;
-  if ((rc = force_begin(c))) return rc;
+  if ((rc = force_begin(c, true))) return rc;
   auto mark = [&]() {
     if (!evs) return;
     cudaEvent_t e;
@@ -714,7 +716,7 @@ static int enqueue_step(solar_ctx* c, const int* runs, std::vector<cudaEvent_t>*
   mark();
   if ((rc = launch_filter<T>(c, bufs[cur], bufs[cur ^ 1], runs))) return rc;
   mark();
-  return force_end(c);
+  return SOLAR_OK;
 }
 
 static int enqueue_step_any(solar_ctx* c, const int* runs, std::vector<cudaEvent_t>* evs) {
@@ -764,6 +766,38 @@ static int watch_after_step(solar_ctx* c) {
   else nonfinite_kernel<double><<<grid, 256, 0, c->stream>>>((const double*)c->A, g, step, c->err + 1);
   CK(cudaGetLastError());
   return SOLAR_OK;
+}
+
+// Sum of squares of one stored field of the state into out[ctl[1]].
+template <typename T>
+static int launch_sumsq(solar_ctx* c, int run, int slot, double* out) {
+  const SumsqArgs<T> a = {(const T*)c->A, c->part, out, c->norm_ctl, c->g, run, slot};
+  CK(launch_pdl(sumsq_kernel<T>, dim3((unsigned)(c->g.nface * (c->g.k1 - c->g.k0))), dim3(256), 0, c->stream, a));
+  return SOLAR_OK;
+}
+
+// The step and the norm's sum of one run and slot (slot < 0: the step alone).
+static int capture_norm_graph(solar_ctx* c, int run, int slot) {
+  if (c->norm_graph && c->norm_run == run && c->norm_slot == slot) return SOLAR_OK;
+  if (c->norm_graph) { cudaGraphExecDestroy(c->norm_graph); c->norm_graph = nullptr; }
+  cudaGraph_t graph;
+  CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+  int rc = enqueue_step_any(c, nullptr, nullptr);
+  if (!rc && slot >= 0) rc = c->fp32 ? launch_sumsq<float>(c, run, slot, c->norm_ring) : launch_sumsq<double>(c, run, slot, c->norm_ring);
+  cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
+  if (rc) return rc;
+  CK(ce);
+  CK(cudaGraphInstantiate(&c->norm_graph, graph, 0));
+  CK(cudaGraphDestroy(graph));
+  c->norm_run = run;
+  c->norm_slot = slot;
+  return SOLAR_OK;
+}
+
+// Captured graphs hold launch shapes and arguments: dropped when those change.
+static void drop_step_graphs(solar_ctx* c) {
+  for (auto* gx : {&c->step_graph, &c->norm_graph})
+    if (*gx) { cudaGraphExecDestroy(*gx); *gx = nullptr; }
 }
 
 static int capture_step_graph(solar_ctx* c) {
@@ -1057,12 +1091,9 @@ static int reduce(solar_ctx* c, int run, int sel_field, double* out5) {
 static int sumsq(solar_ctx* c, int run, int sel_field, double* out) {
   const int s = c->g.slot[sel_field];
   if (s < 0) { *out = 0.0; return SOLAR_OK; }
-  const int nblocks = c->g.nface * (c->g.k1 - c->g.k0);
-  if (c->fp32) sumsq_plane_kernel<float><<<nblocks, 256, 0, c->stream>>>((const float*)c->A, c->g, run, s, c->part);
-  else sumsq_plane_kernel<double><<<nblocks, 256, 0, c->stream>>>((const double*)c->A, c->g, run, s, c->part);
-  CK(cudaGetLastError());
-  sumsq_final_kernel<<<1, 256, 0, c->stream>>>(c->part, nblocks, c->red_out);
-  CK(cudaGetLastError());
+  CK(cudaMemsetAsync(c->norm_ctl, 0, 2 * sizeof(int), c->stream));
+  int rc = c->fp32 ? launch_sumsq<float>(c, run, s, c->red_out) : launch_sumsq<double>(c, run, s, c->red_out);
+  if (rc) return rc;
   CK(cudaMemcpyAsync(out, c->red_out, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   return SOLAR_OK;
@@ -1107,9 +1138,9 @@ int solar_gpu_finalize(solar_ctx* c) {
   if (!c) return SOLAR_OK;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
-  if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
+  drop_step_graphs(c);
   drop_batch_graphs(c);
-  void* ptrs[] = {c->A, c->B, c->W, c->stage64, c->part, c->red_out, c->run_order,
+  void* ptrs[] = {c->A, c->B, c->W, c->stage64, c->part, c->red_out, c->norm_ctl, c->run_order,
                   c->err, c->dt.rad, c->dt.met, c->dt.radT, c->dt.ew, c->dt.eg, c->dt.egc, c->dt.s0t, c->dt.ewin, c->dt.c2,
                   c->dt.rad64, c->dt.vol2, c->dt.drw, c->dt.c2_64, c->dt.tanx, c->dt.gr};
   for (void* p : ptrs)
@@ -1197,6 +1228,8 @@ int solar_gpu_init(const solar_desc* d, solar_ctx** out) {
   TRYC(cudaMalloc((void**)&c->stage64, (size_t)vol_compact(c) * sizeof(double)));
   TRYC(cudaMalloc((void**)&c->part, (size_t)6 * g.nr * 5 * sizeof(double)));
   TRYC(cudaMalloc((void**)&c->red_out, 5 * sizeof(double)));
+  TRYC(cudaMalloc((void**)&c->norm_ctl, 2 * sizeof(int)));
+  TRYC(cudaMemset(c->norm_ctl, 0, 2 * sizeof(int)));
   TRYC(cudaMalloc((void**)&c->run_order, g.nruns * sizeof(int)));
   TRY(upload_constants());
   if (c->fp32) TRY(upload_tables<float>(c));
@@ -1342,7 +1375,7 @@ int solar_gpu_compute_rhs(solar_ctx* c, const double* q, double* rhs) {
   if (rc) return rc;
   if (!q || !rhs) return fail(SOLAR_ERR_ARG, "null array");
   if ((rc = op_prepare_state(c, q))) return rc;
-  if ((rc = force_begin(c))) return rc;
+  if ((rc = force_begin(c, false))) return rc;
   if (c->fp32) { launch_edge<float>(c, c->B, 0, nullptr); rc = launch_stage<float>(c, c->B, c->W, 2, 0, nullptr); }
   else { launch_edge<double>(c, c->B, 0, nullptr); rc = launch_stage<double>(c, c->B, c->W, 2, 0, nullptr); }
   if (rc) return rc;
@@ -1511,6 +1544,7 @@ int solar_gpu_rk4_norms(solar_ctx* c, int run, int field, int nsteps, double* no
   if (nsteps == 0) return SOLAR_OK;
   if (c->norm_ring_len < nsteps) {
     CK(cudaStreamSynchronize(c->stream));
+    if (c->norm_graph) { cudaGraphExecDestroy(c->norm_graph); c->norm_graph = nullptr; }   // holds the old address
     if (c->norm_ring) cudaFree(c->norm_ring);
     c->norm_ring = nullptr;
     c->norm_ring_len = 0;
@@ -1518,18 +1552,13 @@ int solar_gpu_rk4_norms(solar_ctx* c, int run, int field, int nsteps, double* no
     if (e != cudaSuccess) return fail(SOLAR_ERR_NOMEM, "per-step norms: %s", cudaGetErrorString(e));
     c->norm_ring_len = nsteps;
   }
-  if ((rc = capture_step_graph(c))) return rc;
   const int slot = c->g.slot[field - 1];
-  const int nblocks = c->g.nface * (c->g.k1 - c->g.k0);
+  if ((rc = capture_norm_graph(c, run, slot))) return rc;
+  CK(cudaMemsetAsync(c->norm_ctl, 0, 2 * sizeof(int), c->stream));
   if (slot < 0) CK(cudaMemsetAsync(c->norm_ring, 0, (size_t)nsteps * sizeof(double), c->stream));
   for (int s = 0; s < nsteps; ++s) {
-    CK(cudaGraphLaunch(c->step_graph, c->stream));
+    CK(cudaGraphLaunch(c->norm_graph, c->stream));
     if ((rc = watch_after_step(c))) return rc;
-    if (slot < 0) continue;
-    if (c->fp32) sumsq_plane_kernel<float><<<nblocks, 256, 0, c->stream>>>((const float*)c->A, c->g, run, slot, c->part);
-    else sumsq_plane_kernel<double><<<nblocks, 256, 0, c->stream>>>((const double*)c->A, c->g, run, slot, c->part);
-    sumsq_final_kernel<<<1, 256, 0, c->stream>>>(c->part, nblocks, c->norm_ring + s);
-    CK(cudaGetLastError());
   }
   CK(cudaMemcpyAsync(norms, c->norm_ring, (size_t)nsteps * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -1557,7 +1586,7 @@ int solar_gpu_inject_wait_timeout(solar_ctx* c, int kernels, int polls) {
   c->inject_mask = kernels;
   c->inject_polls = kernels ? (uint32_t)polls : 0u;
   // the captured step graphs hold the old launch arguments
-  if (c->step_graph) { cudaGraphExecDestroy(c->step_graph); c->step_graph = nullptr; }
+  drop_step_graphs(c);
   drop_batch_graphs(c);
   return SOLAR_OK;
 }

@@ -61,7 +61,7 @@ static int lines_op(solar_ctx* c, int phase, const int* zone_edge, int count, vo
 template <typename T>
 static int enqueue_phase(solar_ctx* c, int phase) {
   int rc;
-  if (phase == 0 && (rc = force_begin(c))) return rc;
+  if (phase == 0 && (rc = force_begin(c, true))) return rc;
   if (phase < 5) {
     void* in = phase % 2 ? c->B : c->A;
     void* out = phase % 2 ? c->A : c->B;
@@ -70,8 +70,7 @@ static int enqueue_phase(solar_ctx* c, int phase) {
   }
   if (phase != 7 && (rc = launch_edge<T>(c, c->B, 1, nullptr))) return rc;
   if (phase == 6) return SOLAR_OK;
-  if ((rc = launch_filter<T>(c, c->B, c->A, nullptr))) return rc;
-  return force_end(c);
+  return launch_filter<T>(c, c->B, c->A, nullptr);
 }
 
 // Phases 0..4 in two parts, so that a process can overlap the edge-line exchange with
@@ -87,7 +86,7 @@ static int enqueue_phase_part(solar_ctx* c, int phase, int part) {
   void* out = phase % 2 ? c->A : c->B;
   const int mode = phase == 0 ? 1 : 0;
   if (part == 0) {
-    if (phase == 0 && (rc = force_begin(c))) return rc;
+    if (phase == 0 && (rc = force_begin(c, true))) return rc;
     return launch_stage<T>(c, in, out, mode, phase, nullptr, nullptr, kTilesInterior);
   }
   if ((rc = launch_edge<T>(c, in, 0, nullptr))) return rc;
@@ -148,7 +147,7 @@ int solar_gpu_set_owned_zones(solar_ctx* c, int zone0, int nzones) {
   c->g.face0 = zone0;
   c->g.nface = nzones;
   // captured graphs hold the old launch shapes
-  if (c->step_graph) { cudaGraphExecDestroy(c->step_graph); c->step_graph = nullptr; }
+  drop_step_graphs(c);
   drop_batch_graphs(c);
   return SOLAR_OK;
 }
@@ -195,7 +194,7 @@ int solar_gpu_set_owned_planes(solar_ctx* c, int k0, int k1) {
   c->g.k0 = k0;
   c->g.k1 = k1;
   // captured graphs hold the old launch shapes
-  if (c->step_graph) { cudaGraphExecDestroy(c->step_graph); c->step_graph = nullptr; }
+  drop_step_graphs(c);
   drop_batch_graphs(c);
   return SOLAR_OK;
 }

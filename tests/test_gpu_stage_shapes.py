@@ -92,3 +92,23 @@ def test_batch_shapes_follow_the_live_runs(oracle_mod):
             got, want = s.get_state(r), o.rk4(q[r], n)
             for m in range(5):
                 assert rel_l2(got[:, m], want[:, m]) <= 1e-11, (r, m)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_norms_across_runs_fields_and_lengths(precision):
+    """The norm is part of the step graph: a change of run or field, a longer ring, an unstored
+    field and calls of solar_gpu_norm in between give the norms of single steps, bit for bit."""
+    cfg = configs.c2(nx=32, nr=21)
+    q = np.random.default_rng(5).standard_normal((2, 6, 5, 21, 32, 32))
+    calls = [(0, 4, 2), (0, 4, 3), (1, 4, 2), (1, 5, 6), (0, 1, 1), (0, 2, 4)]
+    with Solver(cfg, precision=precision, nfields=4, nruns=2) as s, Solver(cfg, precision=precision, nfields=4, nruns=2) as o:
+        for r in range(2):
+            s.set_state(q[r], r)
+            o.set_state(q[r], r)
+        for run, field, n in calls:
+            want = []
+            for _ in range(n):
+                o.rk4(1)
+                want.append(o.norm(field, run))
+            np.testing.assert_array_equal(s.rk4_norms(n, field, run), want)
+            assert s.norm(field, run) == want[-1]
