@@ -4,6 +4,7 @@
 #include <cudaTypedefs.h>
 
 #include <sched.h>
+#include <sys/mman.h>
 
 #include <algorithm>
 #include <cmath>
@@ -165,7 +166,8 @@ struct AdjBuffers {
 using namespace solar;
 
 constexpr int kStageBlocks = 8;
-constexpr size_t kStageBytes = 4u << 20;
+constexpr size_t kStageBytes = 2u << 20;
+constexpr size_t kStageMap = (kStageBlocks + 1) * kStageBytes;   // room to align the blocks
 
 struct solar_ctx {
   solar_desc desc;
@@ -208,7 +210,8 @@ struct solar_ctx {
   cudaEvent_t xev[2] = {};
   std::unique_ptr<HostPool> pool;
   // Pageable arrays of the caller move through kStageBlocks pinned blocks (on first use).
-  char* pin_stage = nullptr;
+  char* pin_stage = nullptr;   // inside the mapping pin_map
+  void* pin_map = nullptr;
   cudaEvent_t sev[kStageBlocks] = {};
   AdjBuffers adj;
   int forcing = 0;             // SOLAR_FORCING_*
@@ -864,27 +867,44 @@ static void slice(long long n, int t, int p, long long* lo, long long* hi) {
   *hi = n * (t + 1) / p;
 }
 
-// Whether an array of the caller, moved in volumes of `bytes`, goes through the pinned blocks:
-// pageable memory in volumes of at least 1 MiB.  The driver moves such arrays through a staging
-// buffer of its own with one thread, which also takes the page faults of a fresh result array
-// (COMPUTE_RHS at 6 x 64^3 in double, 63 MB out into fresh memory: 16.2 ms, now 6.3; at 6 x 96^3
-// 50 ms, now 18; a pageable state in at 6 x 96^3 19.4 ms, now 7.0).  Smaller volumes do not
-// repay waking the threads (6 x 48^3, 0.9 MB each: the same 3.2 ms).
-static bool stage_pageable(const void* p, size_t bytes) {
-  if (bytes < (1u << 20)) return false;
-  cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return false; }
-  return at.type == cudaMemoryTypeUnregistered;
-}
-
+// The pinned blocks, their events and the host threads, on first use.
 static int ensure_stage(solar_ctx* c) {
   if (c->pin_stage) return SOLAR_OK;
   int rc;
   if ((rc = ensure_pool(c))) return rc;
   for (auto& e : c->sev)
     if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  CK(cudaHostAlloc((void**)&c->pin_stage, kStageBlocks * kStageBytes, cudaHostAllocDefault));
+  // Huge pages registered with the driver: a context's first transfer pays for its blocks, and
+  // 16 MB take 2.9 ms this way, 10 ms with cudaHostAlloc.
+  if (!c->pin_map) {
+    void* m = mmap(nullptr, kStageMap, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS, -1, 0);
+    if (m == MAP_FAILED) return fail(SOLAR_ERR_NOMEM, "staging blocks: mmap failed");
+    c->pin_map = m;
+  }
+  char* p = (char*)(((uintptr_t)c->pin_map + kStageBytes - 1) / kStageBytes * kStageBytes);
+  madvise(p, kStageBlocks * kStageBytes, MADV_HUGEPAGE);      // a hint: small pages work as well
+  c->pool->run([&](int t) {
+    for (int b = t; b < kStageBlocks; b += c->pool->size()) std::memset(p + b * kStageBytes, 0, kStageBytes);
+  });
+  CK(cudaHostRegister(p, kStageBlocks * kStageBytes, cudaHostRegisterDefault));
+  c->pin_stage = p;
   return SOLAR_OK;
+}
+
+// Whether an array of the caller, moved in volumes of `bytes`, goes through the pinned blocks:
+// pageable memory in volumes of at least 1 MiB.  The driver moves such arrays through a staging
+// buffer of its own with one thread, which also takes the page faults of a fresh result array
+// (COMPUTE_RHS at 6 x 64^3 in double, 63 MB out into fresh memory: 16.2 ms, now 6.3; at 6 x 96^3
+// 50 ms, now 18; a pageable state in at 6 x 96^3 19.4 ms, now 7.0).  Smaller volumes do not
+// repay waking the threads (6 x 48^3, 0.9 MB each: the same 3.2 ms).
+static bool stage_pageable(solar_ctx* c, const void* p, size_t bytes) {
+  if (bytes < (1u << 20)) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return false; }
+  if (at.type != cudaMemoryTypeUnregistered) return false;
+  if (ensure_stage(c) == SOLAR_OK) return true;
+  cudaGetLastError();                                    // no pinned memory or threads: copy as it is
+  return false;
 }
 
 // Copies between the device and a pageable array, on the context's stream, through the pinned
@@ -898,7 +918,6 @@ class Staged {
   explicit Staged(solar_ctx* c) : c_(c) {}
   int out(void* host, const void* dev, size_t bytes) {
     int rc;
-    if ((rc = ensure_stage(c_))) return rc;
     for (size_t o = 0; o < bytes; o += kStageBytes) {
       if (head_ - tail_ == kStageBlocks && (rc = drain(kStageBlocks / 2))) return rc;
       const int s = (int)(head_ % kStageBlocks);
@@ -918,8 +937,6 @@ class Staged {
     return SOLAR_OK;
   }
   int in(void* dev, const void* host, size_t bytes) {
-    int rc;
-    if ((rc = ensure_stage(c_))) return rc;
     for (size_t o = 0; o < bytes; o += kStageBytes) {
       const int s = (int)(head_ % kStageBlocks);
       const size_t n = std::min(kStageBytes, bytes - o);
@@ -1004,7 +1021,7 @@ static int upload_fields(solar_ctx* c, void* buf, int run, const double* host, i
   if (c->fp32) return upload_fields32(c, buf, run, host, nh, fields, nfields_h);
   const long long V = vol_compact(c);
   const size_t bytes = (size_t)V * sizeof(double);
-  const bool staged = stage_pageable(host, bytes);
+  const bool staged = stage_pageable(c, host, bytes);
   Staged st(c);
   const int threads = 256;
   const int blocks = (int)((V + threads - 1) / threads);
@@ -1032,7 +1049,7 @@ static int download_fields(solar_ctx* c, const void* buf, int run, double* host,
                            const int* fields, int nfields_h) {
   const long long V = vol_compact(c);
   const size_t bytes = (size_t)V * sizeof(double);
-  const bool staged = stage_pageable(host, bytes);
+  const bool staged = stage_pageable(c, host, bytes);
   Staged st(c);
   int rc;
   const int threads = 256;
@@ -1157,7 +1174,8 @@ int solar_gpu_finalize(solar_ctx* c) {
   for (auto& e : c->sev)
     if (e) cudaEventDestroy(e);
   if (c->pin32) cudaFreeHost(c->pin32);
-  if (c->pin_stage) cudaFreeHost(c->pin_stage);
+  if (c->pin_stage) cudaHostUnregister(c->pin_stage);
+  if (c->pin_map) munmap(c->pin_map, kStageMap);
   c->pool.reset();
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
