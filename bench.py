@@ -522,11 +522,12 @@ def main():
     # per-kernel launch times (graph off) for the roofline of the dominant kernel
     kt = s32.time_rk4(max(4, min(args.steps, 20)), per_kernel=True)
     F, w = 4, 4
-    stage_bytes = (3 * F + 4 * 4 * F) / 5.0 * w * pts          # mean algorithmic bytes per stage launch
+    # mean algorithmic bytes per stage launch: stage 1 does not read qw, stage 5 does not write it
+    stage_bytes = (3 * F + 3 * 4 * F + 3 * F) / 5.0 * w * pts
     filter_bytes = 2 * F * w * pts
     stage_gbs = stage_bytes / (kt["stage_ms"] / 1e3) / 1e9
     filter_gbs = filter_bytes / (kt["filter_ms"] / 1e3) / 1e9
-    step_bytes = 21 * F * w * pts
+    step_bytes = 20 * F * w * pts
     s32.close()
 
     # ---------------------------------------------------------------- FP64 plain path
@@ -592,8 +593,8 @@ def main():
                      "mean_launch_ms": kt["stage_ms"],
                      "filter": {"achieved": filter_gbs, "frac": filter_gbs / peak, "mean_launch_ms": kt["filter_ms"]},
                      "edge_mean_launch_ms": kt["edge_ms"],
-                     "step_roofline_pt_steps_per_s": peak * 1e9 / (21 * F * w),
-                     "step_frac": (value / world) * (21 * F * w) / (peak * 1e9)},
+                     "step_roofline_pt_steps_per_s": peak * 1e9 / (20 * F * w),
+                     "step_frac": (value / world) * (20 * F * w) / (peak * 1e9)},
         "gpu_launches": 12 * args.steps,
         "clocks": clocks,
         "e2e": e2e,

@@ -940,7 +940,7 @@ class Staged {
     for (size_t o = 0; o < bytes; o += kStageBytes) {
       const int s = (int)(head_ % kStageBlocks);
       const size_t n = std::min(kStageBytes, bytes - o);
-      if (head_ >= kStageBlocks) CK(cudaEventSynchronize(c_->sev[s]));
+      CK(cudaEventSynchronize(c_->sev[s]));              // its last copy, maybe of the upload before this one
       HostPool& pool = *c_->pool;
       pool.run([&](int t) { copy_slice(block(s), (const char*)host + o, n, t, pool.size()); });
       CK(cudaMemcpyAsync((char*)dev + o, block(s), n, cudaMemcpyHostToDevice, c_->stream));

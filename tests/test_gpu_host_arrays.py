@@ -47,3 +47,23 @@ def test_operator_and_gradient_outputs():
         assert s.lib.solar_gpu_misfit_gradient(s._h, 2, 2, ptr(data), None, ptr(b), None, None) == 0
     assert np.linalg.norm(a) > 0
     assert np.linalg.norm(a - b) <= 1e-12 * np.linalg.norm(a)           # atomics reorder sums
+
+
+def test_two_uploads_in_one_call():
+    """SPONGE uploads two states without a wait in between: the second must not overwrite pinned
+    blocks that the first is still being copied out of."""
+    cfg = configs.c1(nx=64, nr=48)
+    rng = np.random.default_rng(3)
+    q, rhs = rng.standard_normal((2, 6, 5, 48, 64, 64))
+    qp = pinned(q.shape)
+    qp[...] = q
+    with Solver(cfg) as s:
+        want = s.sponge(qp, rhs)
+        for _ in range(5):
+            np.testing.assert_array_equal(s.sponge(q, rhs), want)
+    # v_xi and v_eta are not damped, the others by sigma(k) q (values of a few units: one rounding)
+    np.testing.assert_array_equal(want[:, 1:3], rhs[:, 1:3])
+    sigma = np.median((rhs - want)[:, 4] / q[:, 4], axis=(0, 2, 3))
+    assert sigma.max() > 0.08
+    for m in (0, 3, 4):
+        assert np.abs(rhs[:, m] - sigma[None, :, None, None] * q[:, m] - want[:, m]).max() <= 1e-14
