@@ -996,7 +996,7 @@ static int upload_fields32(solar_ctx* c, void* buf, int run, const double* host,
       const int s = c->g.slot[fields[m]];
       if (s < 0) continue;
       const int b = q & 1;
-      if (q >= 2) CK(cudaEventSynchronize(c->xev[b]));       // the copy out of block b is done
+      CK(cudaEventSynchronize(c->xev[b]));                   // its last copy, maybe of the upload before this one
       const double* src = host + ((long long)z * nh + m) * V;
       float* pin = c->pin32 + b * V;
       pool.run([&](int t) {
