@@ -43,8 +43,9 @@ namespace solar {
 // coefficient-weighted volumes X1, X2 (on the tile and its xi halo) and Y1, Y2 (tile and eta
 // halo) in shared memory (zero outside the face and on the BC planes; every thread takes its
 // own vector and at most one halo vector), and after one barrier applies -D_xi / -D_eta.  The
-// exchange arrays are double-buffered and a slot is read before the barrier only, so that one
-// barrier per plane serves both and thread 0 refills the slot right after it.  The banded
+// exchange arrays are double-buffered and a slot is read before the barrier only (behind a fence:
+// most of what is read stays in registers), so that one barrier per plane serves both and thread 0
+// refills the slot right after it.  The banded
 // radial transpose adds each plane's facr * R1, facr * R2 to the partial outputs of the planes
 // m-3 .. m+3, held in registers; a plane is complete three iterations later.  The one-sided
 // rows of the radial stencil (planes 1, 2, nr-3, nr-2; planes 0 and nr-1 carry zero) reach the
@@ -389,6 +390,7 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
           if (mu_face) stv(mu_face + sRho * vs + o, nrho);
         }
         // every thread is done with the slot and has written its exchange vectors
+        fence_reads_before_copies();
         if (__syncthreads_or(!ok)) { failed = true; break; }
         if (tid == 0 && loads && m_issued <= m_hi) issue(m_issued++, slot);
         T w1[NV * V], w2[NV * V];
@@ -468,6 +470,7 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
           }
         }
       } else {
+        fence_reads_before_copies();
         if (__syncthreads_or(!ok)) { failed = true; break; }
         if (tid == 0 && loads && m_issued <= m_hi) issue(m_issued++, slot);
       }

@@ -57,6 +57,15 @@ __device__ __forceinline__ void mbar_fence_init() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Before the CTA barrier behind which a ring slot is refilled: this thread's reads of the slot come
+// before the copies that overwrite it.  A barrier alone orders reads only against other threads'
+// ordinary accesses; the copies go through another proxy, and a read whose value is first used
+// after the barrier may still be under way when they are issued.  Not needed where every value
+// read feeds a store in front of the barrier.
+__device__ __forceinline__ void fence_reads_before_copies() {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
                : "memory");
