@@ -84,6 +84,20 @@ struct AdjStageArgs {
 // for the one-sided rows) took 2163 and 1198.
 constexpr int kAdjRing = 2;
 
+// Rounding.  dt L^T(mu) is small against lambda_q, so its terms are summed up before lambda_q comes
+// in wherever registers allow, and what has to be added to the large sum later is added in as few
+// parts as possible.  Error of lambda after 1 / 20 reverse steps in float against double, 6 x 48^2 x
+// 33, 6 x 96^3: 1.12e-7 / 2.84e-7, 1.20e-7 / 3.23e-7; with lambda_q first and every plane's radial
+// term added to it by itself 1.53e-7 / 3.42e-7, 1.65e-7 / 4.15e-7.  In float lambda_q of p, v_xi and
+// v_eta waits for the terms behind the barrier, and a plane's radial term of p for the next plane's
+// (a step takes 0.3% less with four fields, 2.6% less with five, mean over ten grids from 6 x 64^3
+// to 6 x 128^3).  In double the registers are used up: the same costs 5-30%, so there lambda_q
+// comes in with the pointwise terms and the three later radial terms one by one.
+template <typename T>
+struct AdjSums {
+  static constexpr bool late = sizeof(T) == 4;
+};
+
 template <typename T, int TX, int TY, bool HAS_RHO>
 struct AdjLayout {
   static constexpr int V = Vec16<T>::V, NTH = TX / V * TY;
@@ -103,7 +117,8 @@ struct AdjLayout {
   static constexpr size_t EX = kAdjRing * SLOT;                     // [2][X1, X2, Y1, Y2]
   static constexpr size_t EX_BYTES = 2 * (XB + YB) * sizeof(T);
   static constexpr size_t ONE = EX + 2 * EX_BYTES;                  // one-sided rows, [4][NTH] vectors
-  static constexpr size_t BAR = ONE + (size_t)4 * NTH * 16;
+  static constexpr size_t HELD = ONE + (size_t)4 * NTH * 16;        // a plane's radial term of p (AdjSums)
+  static constexpr size_t BAR = HELD + (AdjSums<T>::late ? (size_t)NTH * 16 : 0);
   static constexpr size_t TOTAL = BAR + kAdjRing * sizeof(uint64_t);
 };
 
@@ -114,6 +129,7 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
   constexpr int QV = 4 / V;                          // vectors in the 4-column margin of a box
   constexpr int NETA = 6 * NT, NXI = 2 * QV * TY;    // halo vectors
   constexpr int NV = (V + 8) / V;                    // vectors covering columns c-4 .. c+V+3
+  constexpr bool LATE = AdjSums<T>::late;
   constexpr int PBs = L::PB, OBs = L::OB, R0 = HAS_RHO ? 1 : 0;   // storage slots: (rho,) v_xi, v_eta, v_r, p
   static_assert(NETA + NXI <= L::NTH, "one halo vector per thread");
   extern __shared__ __align__(128) unsigned char smem[];
@@ -223,7 +239,7 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       const T c2rho0 = tc2 ? cc[q] * rho0 : rr[rC2Rho0];
-      r1[q] = -f * rr[rInvRho0] * (a.beta * vv[q]);
+      r1[q] = f * (-rr[rInvRho0] * (a.beta * vv[q]));
       r2[q] = -f * (c2rho0 * (a.beta * vp[q]) + (HAS_RHO ? rho0 * (a.beta * vrho[q]) : T(0)));
     }
     T* d = reinterpret_cast<T*>(smem + L::ONE) + (size_t)tid * V;
@@ -241,6 +257,8 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
 #pragma unroll
     for (int d = 0; d < 4; ++d) { kp[d][q] = T(0); kv[d][q] = T(0); }
   }
+  T* const held = reinterpret_cast<T*>(smem + L::HELD) + (size_t)tid * V;   // only with LATE
+  if constexpr (LATE) stv(held, ap[0]);
   int slot = 0;
   uint32_t phase = 0;
   bool ok = true, failed = false;
@@ -281,13 +299,20 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
         e[q] = bc ? T(0) : -c2rho0 * mP[q] - (HAS_RHO ? rho0 * mRho[q] : T(0));
       }
       // banded radial transpose (rows 3 .. nr-4): plane m reaches the planes m-3 .. m+3
-      if (m >= 3 && m <= nr - 4) {
-        const T f = a.dt * rr[rFacR];
+      if (LATE || (m >= 3 && m <= nr - 4)) {
+        const T f = (m >= 3 && m <= nr - 4) ? a.dt * rr[rFacR] : T(0);
+        T w1[V], wl[V];                            // of plane m; of plane m-1 where it was held
+        if constexpr (LATE) ldv(held, wl);
+#pragma unroll
+        for (int q = 0; q < V; ++q) w1[q] = f * (-inv_rho0 * mR[q]);
+        if constexpr (LATE) stv(held, w1);
 #pragma unroll
         for (int q = 0; q < V; ++q) {
-          const T w1 = -f * inv_rho0 * mR[q], w2 = f * e[q];
-          ap[0][q] -= c3 * w1; ap[1][q] -= c2c * w1; ap[2][q] -= c1 * w1;
-          ap[4][q] += c1 * w1; ap[5][q] += c2c * w1; ap[6][q] += c3 * w1;
+          const T w2 = f * e[q];
+          ap[0][q] -= c3 * w1[q];
+          if constexpr (LATE) ap[1][q] -= c1 * wl[q] + c2c * w1[q];
+          else { ap[1][q] -= c2c * w1[q]; ap[2][q] -= c1 * w1[q]; }
+          ap[4][q] += c1 * w1[q]; ap[5][q] += c2c * w1[q]; ap[6][q] += c3 * w1[q];
           av[0][q] -= c3 * w2; av[1][q] -= c2c * w2; av[2][q] -= c1 * w2;
           av[4][q] += c1 * w2; av[5][q] += c2c * w2; av[6][q] += c3 * w2;
         }
@@ -372,12 +397,15 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
             orho[q] = (a.keep ? lRho[q] : T(0)) + a.dt * (-rr[rG0Rho0] * pr - sig * mRho[q]);
             nrho[q] = a.alpha * mRho[q] + a.beta_next * orho[q];
           }
-          ap[3][q] += (a.keep ? lP[q] : T(0)) - a.dt * sig * mP[q];
-          av[3][q] += (a.keep ? lR[q] : T(0)) + a.dt * vr_;
+          ap[3][q] -= a.dt * sig * mP[q];
+          if constexpr (!LATE) ap[3][q] = (a.keep ? lP[q] : T(0)) + ap[3][q];
+          av[3][q] = (a.keep ? lR[q] : T(0)) + (av[3][q] + a.dt * vr_);
           kp[3][q] = a.alpha * mP[q];
           kv[3][q] = a.alpha * mR[q];
-          lX[q] = (a.keep ? lX[q] : T(0)) - a.dt * (invr * gTX[q] * e[q]);
-          lE[q] = (a.keep ? lE[q] : T(0)) - a.dt * (invr * gTY[q] * e[q]);
+          if constexpr (!LATE) {
+            lX[q] = (a.keep ? lX[q] : T(0)) - a.dt * (invr * gTX[q] * e[q]);
+            lE[q] = (a.keep ? lE[q] : T(0)) - a.dt * (invr * gTY[q] * e[q]);
+          }
           if (tdiv) gacc[q] += (double)(a.dt * (rho0 * div[q]) * pp);
         }
         if (tdiv) {
@@ -423,9 +451,15 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
         for (int q = 0; q < V; ++q) {
           d1[q] += dxi(w1, 4 + q);
           d2[q] = dxi(w2, 4 + q);
-          ap[3][q] += k2 * d1[q];
-          lX[q] += k2 * d2[q];
-          lE[q] += k2 * dy2[q];
+          if constexpr (LATE) {
+            ap[3][q] = (a.keep ? lP[q] : T(0)) + (ap[3][q] + k2 * d1[q]);
+            lX[q] = (a.keep ? lX[q] : T(0)) + (k2 * d2[q] - a.dt * (invr * gTX[q] * e[q]));
+            lE[q] = (a.keep ? lE[q] : T(0)) + (k2 * dy2[q] - a.dt * (invr * gTY[q] * e[q]));
+          } else {
+            ap[3][q] += k2 * d1[q];
+            lX[q] += k2 * d2[q];
+            lE[q] += k2 * dy2[q];
+          }
           nX[q] = a.alpha * mX[q] + a.beta_next * lX[q];
           nE[q] = a.alpha * mE[q] + a.beta_next * lE[q];
         }
@@ -475,6 +509,15 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
         if (tid == 0 && loads && m_issued <= m_hi) issue(m_issued++, slot);
       }
       if (++slot == kAdjRing) { slot = 0; phase ^= 1; }
+    } else if constexpr (LATE) {                   // beside the shell: only the held term
+      T wl[V];
+      ldv(held, wl);
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        ap[1][q] -= c1 * wl[q];
+        wl[q] = T(0);
+      }
+      stv(held, wl);
     }
     const int pl = m - 3;
     if (pl >= kb && pl < ke) {
@@ -482,6 +525,7 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
         const bool low = pl < 7;
         if (!low && pl == max(kb, nr - 7)) { one_sided(nr - 3, 0); one_sided(nr - 2, 1); }
         const T* d = reinterpret_cast<const T*>(smem + L::ONE) + (size_t)tid * V;
+        T s1[V], s2[V];
 #pragma unroll
         for (int row = 0; row < 2; ++row) {
           const T b = low ? Coef<T>::bdy(1 + row, pl) : -Coef<T>::bdy(2 - row, nr - 1 - pl);
@@ -489,8 +533,13 @@ __global__ void __launch_bounds__(TX / Vec16<T>::V * TY) adj_stage_kernel(const 
           ldv(d + (2 * row) * L::NTH * V, r1);
           ldv(d + (2 * row + 1) * L::NTH * V, r2);
 #pragma unroll
-          for (int q = 0; q < V; ++q) { ap[0][q] += b * r1[q]; av[0][q] += b * r2[q]; }
+          for (int q = 0; q < V; ++q) {
+            s1[q] = row ? s1[q] + b * r1[q] : b * r1[q];
+            s2[q] = row ? s2[q] + b * r2[q] : b * r2[q];
+          }
         }
+#pragma unroll
+        for (int q = 0; q < V; ++q) { ap[0][q] += s1[q]; av[0][q] += s2[q]; }
       }
       const int op = pl * plane + own0;
       stv(lo_face + sP * vs + op, ap[0]);
@@ -642,7 +691,10 @@ __global__ void adj_edge_kernel(const __grid_constant__ AdjEdgeArgs<T> a) {
 // then xi^T; the three act along different axes, so they commute and the radial one can come
 // last, on a register queue as in filter_kernel: per plane the xi and eta filters with zero
 // halos (the tensor map covers the interior only, so the load fills them), then the 11-point
-// radial filter over the planes [5, nr-6] (the forward output is zero outside them).  Tiles,
+// radial filter over the planes [5, nr-6] (the forward output is zero outside them).  Every sum runs
+// from the outer taps to the centre: the rounding of a sum counts where it is large, and the radial
+// filter, being last, is followed by none that smooths it (error in float 4.8e-8; centre first
+// 8.4e-8, with the radial filter first and the xi filter last 7.5e-8; the same time).  Tiles,
 // threads, ring and work split are those of filter_kernel, and so is what bounds it.  us per
 // launch at 6 x 96^3 in double / float: 116 / 54, with adj_ghost_kernel's 42 / 29 beside it (as a
 // radial pass over the whole buffer and a plane-marching xi/eta pass with plain loads, ghost
@@ -697,7 +749,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 
     for (int m = 0; m < NV; ++m) ldv(bx + r * PW + V * cx + m * V, w + m * V);
 #pragma unroll
     for (int q = 0; q < V; ++q)
-      v[q] = f0 * w[4 + q] + f1 * (w[3 + q] + w[5 + q]) + f2 * (w[2 + q] + w[6 + q]) + f3 * (w[1 + q] + w[7 + q]);
+      v[q] = f3 * (w[1 + q] + w[7 + q]) + f2 * (w[2 + q] + w[6 + q]) + f1 * (w[3 + q] + w[5 + q]) + f0 * w[4 + q];
   };
   // radial queue of eta-filtered planes, in float as packed pairs (filter_kernel)
   T tq[11][R][V];
@@ -752,16 +804,16 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 
 #pragma unroll
             for (int h = 0; h < NP; ++h) {
               auto pr = [&](int m) { return pk2(c[r + m][2 * h], c[r + m][2 * h + 1]); };
-              unsigned long long t = mul2(pk2(f0, f0), pr(3));
-              t = fma2(pk2(f1, f1), add2(pr(2), pr(4)), t);
+              unsigned long long t = mul2(pk2(f3, f3), add2(pr(0), pr(6)));
               t = fma2(pk2(f2, f2), add2(pr(1), pr(5)), t);
-              tq2[u][r][h] = fma2(pk2(f3, f3), add2(pr(0), pr(6)), t);
+              t = fma2(pk2(f1, f1), add2(pr(2), pr(4)), t);
+              tq2[u][r][h] = fma2(pk2(f0, f0), pr(3), t);
             }
           } else {
 #pragma unroll
             for (int q = 0; q < V; ++q)
-              tq[u][r][q] = f0 * c[r + 3][q] + f1 * (c[r + 2][q] + c[r + 4][q]) + f2 * (c[r + 1][q] + c[r + 5][q]) +
-                            f3 * (c[r][q] + c[r + 6][q]);
+              tq[u][r][q] = f3 * (c[r][q] + c[r + 6][q]) + f2 * (c[r + 1][q] + c[r + 5][q]) +
+                            f1 * (c[r + 2][q] + c[r + 4][q]) + f0 * c[r + 3][q];
           }
         }
       }
@@ -773,22 +825,22 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 
           if constexpr (PAIRS) {
 #pragma unroll
             for (int h = 0; h < NP; ++h) {
-              unsigned long long acc = mul2(pk2(rw[0], rw[0]), tq2[(u + 6) % 11][r][h]);
+              unsigned long long acc = mul2(pk2(rw[5], rw[5]), add2(tq2[(u + 1) % 11][r][h], tq2[(u + 11) % 11][r][h]));
 #pragma unroll
-              for (int m = 1; m <= 5; ++m)
+              for (int m = 4; m >= 1; --m)
                 acc = fma2(pk2(rw[m], rw[m]), add2(tq2[(u + 6 - m) % 11][r][h], tq2[(u + 6 + m) % 11][r][h]), acc);
               float x, y;
-              upk2(acc, x, y);
+              upk2(fma2(pk2(rw[0], rw[0]), tq2[(u + 6) % 11][r][h], acc), x, y);
               v[2 * h] = x;
               v[2 * h + 1] = y;
             }
           } else {
 #pragma unroll
             for (int q = 0; q < V; ++q) {
-              T acc = rw[0] * tq[(u + 6) % 11][r][q];
+              T acc = rw[5] * (tq[(u + 1) % 11][r][q] + tq[(u + 11) % 11][r][q]);
 #pragma unroll
-              for (int m = 1; m <= 5; ++m) acc += rw[m] * (tq[(u + 6 - m) % 11][r][q] + tq[(u + 6 + m) % 11][r][q]);
-              v[q] = acc;
+              for (int m = 4; m >= 1; --m) acc += rw[m] * (tq[(u + 6 - m) % 11][r][q] + tq[(u + 6 + m) % 11][r][q]);
+              v[q] = acc + rw[0] * tq[(u + 6) % 11][r][q];
             }
           }
           stv(out + (long long)(k - 5) * g.plane + r * g.pitch, v);
@@ -856,11 +908,10 @@ __global__ void __launch_bounds__(128) adj_ghost_kernel(const __grid_constant__ 
 #pragma unroll
     for (int l = 0; l < 3; ++l) {
       const T x = e == 2 ? u[l] : u[3 - l];
-      T s = f0 * x;
-      s += f1 * (__shfl_up_sync(0xffffffffu, x, 1) + __shfl_down_sync(0xffffffffu, x, 1));
+      T s = f3 * (__shfl_up_sync(0xffffffffu, x, 3) + __shfl_down_sync(0xffffffffu, x, 3));
       s += f2 * (__shfl_up_sync(0xffffffffu, x, 2) + __shfl_down_sync(0xffffffffu, x, 2));
-      s += f3 * (__shfl_up_sync(0xffffffffu, x, 3) + __shfl_down_sync(0xffffffffu, x, 3));
-      v[l] = s;
+      s += f1 * (__shfl_up_sync(0xffffffffu, x, 1) + __shfl_down_sync(0xffffffffu, x, 1));
+      v[l] = s + f0 * x;
     }
   };
   T q[11][3];
@@ -870,9 +921,10 @@ __global__ void __launch_bounds__(128) adj_ghost_kernel(const __grid_constant__ 
     T s[3];
 #pragma unroll
     for (int l = 0; l < 3; ++l) {
-      s[l] = rw[0] * q[5][l];
+      s[l] = rw[5] * (q[0][l] + q[10][l]);
 #pragma unroll
-      for (int d = 1; d <= 5; ++d) s[l] += rw[d] * (q[5 - d][l] + q[5 + d][l]);
+      for (int d = 4; d >= 1; --d) s[l] += rw[d] * (q[5 - d][l] + q[5 + d][l]);
+      s[l] += rw[0] * q[5][l];
     }
     const T w[3] = {f1 * s[0] + f2 * s[1] + f3 * s[2], f2 * s[0] + f3 * s[1], f3 * s[0]};   // layers 1, 2, 3
     if (writes) {
