@@ -734,9 +734,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 
     mbar_fence_init();
   }
   __syncthreads();
-  // No wait here: adj_ghost_kernel, launched before this one, releases it only after its own wait,
-  // so the kernels before that one are complete; the two run side by side (this one waits at
-  // its end).
+  grid_dependency_wait();
   const bool loads = !a.wc.no_loads;
   if (tid == 0 && loads)
     for (int k = ks; k < min(ks + kFiltRing, ke); ++k) issue(k, k - ks);
@@ -774,6 +772,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 
     for (int u = 0; u < 11; ++u) {
       const int k = kb + u;
       if (k >= ke) break;
+      if (k == ke - release_planes(ke - ks)) release_dependents();
       {
         const bool got = mbar_wait(&bars[slot], phase, a.wc, kErrAdjointRing);
         const T* bx = reinterpret_cast<const T*>(smem + slot * L::P_BYTES);
@@ -853,7 +852,6 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 
     const int k = fail_at >> 1;
     mbar_drain(bars, kFiltRing, ks, k + (fail_at & 1), min(k + kFiltRing, ke), a.wc.polls);
   }
-  grid_dependency_wait();
 }
 
 // Ghost adjoints of FILTER_EXP^T, from the interior of `in` into the frame of `out`.  The eta
@@ -888,7 +886,7 @@ __global__ void __launch_bounds__(128) adj_ghost_kernel(const __grid_constant__ 
   const int t = cols ? gw * 26 + lane - 3 : (int)(blockIdx.x * blockDim.x + threadIdx.x);   // row or column
   const bool in_face = t >= 0 && t < n, writes = in_face && (!cols || (lane >= 3 && lane < 29));
   grid_dependency_wait();
-  release_dependents();                                      // after the wait: adj_filter_kernel relies on it
+  release_dependents();
   if (cols ? gw * 26 >= n : t >= n) return;                  // whole warps (columns) or lone threads
   // the three values next to the edge of plane k, nearest first (eta-filtered for the columns)
   auto load = [&](int k, T* v) {
