@@ -152,7 +152,7 @@ static int launch_adj_filter(solar_ctx* c) {
   using L = FilterLayout<T, TX, TY>;
   AdjBuffers& b = c->adj;
   const Geom& g = c->g;
-  FilterArgs<T> a;
+  FilterArgs<T> a = {};
   if (!make_interior_map(c, b.L, TX + 8, TY + 6, &a.mP)) return fail(SOLAR_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   a.qout = (T*)b.T1;
   a.runs = nullptr;
@@ -220,14 +220,14 @@ static int enqueue_step_div(solar_ctx* c, T* dstep) {
   void* bufs[2] = {c->A, c->B};
   const long long V6 = 6 * vol_compact(c);
   int cur = 0, rc;
-  if ((rc = force_begin(c, true))) return rc;
+  if ((rc = force_begin(c))) return rc;
   for (int s = 0; s < 5; ++s) {
     if ((rc = launch_edge<T>(c, bufs[cur], 0, nullptr))) return rc;
     if ((rc = launch_stage<T>(c, bufs[cur], bufs[cur ^ 1], s == 0 ? 4 : 5, s, nullptr, dstep + s * V6))) return rc;
     cur ^= 1;
   }
   if ((rc = launch_edge<T>(c, bufs[cur], 1, nullptr))) return rc;
-  if ((rc = launch_filter<T>(c, bufs[cur], bufs[cur ^ 1], nullptr))) return rc;
+  if ((rc = launch_filter<T>(c, bufs[cur], bufs[cur ^ 1], nullptr, true))) return rc;
   CK(cudaGetLastError());
   return SOLAR_OK;
 }

@@ -12,8 +12,8 @@
 // timestep.f90:82).  A one-thread clock kernel at the start of each step evaluates the
 // time factors (including the reference's coefficient refresh when floor(xt) advances),
 // a field kernel forms this step's S(x, y) for all faces, the stage kernel adds S(x, y)
-// times the radial factor to the v_r right-hand side; the field kernel advances time and step
-// for the next one.
+// times the radial factor to the v_r right-hand side; the filter kernel, which ends a step,
+// advances time and step.
 #pragma once
 
 namespace solar {
@@ -76,21 +76,17 @@ __global__ void force_clock_kernel(const __grid_constant__ ForceClockArgs a) {
 
 template <typename T>
 struct ForceFieldArgs {
-  ForceClock* c;
+  const ForceClock* c;
   int kind;
   const double* exy;
   const double* samples;
   long long n6;
   T* out;
-  double dt;
-  int advance;              // the step's time += dt, step += 1
 };
 
-// The field does not depend on the time and step words, so one thread advances them for the
-// next step here (a kernel of its own after the filter cost 3 us a step).
 template <typename T>
 __global__ void force_field_kernel(const __grid_constant__ ForceFieldArgs<T> a) {
-  ForceClock* const c = a.c;
+  const ForceClock* const c = a.c;
   const int kind = a.kind;
   const double* exy = a.exy;
   const double* samples = a.samples;
@@ -100,10 +96,6 @@ __global__ void force_field_kernel(const __grid_constant__ ForceFieldArgs<T> a) 
   grid_dependency_wait();
   release_dependents();
   if (p >= n6) return;
-  if (p == 0 && a.advance) {
-    c->time = c->time + a.dt;
-    c->step = c->step + 1;
-  }
   if (kind == SOLAR_FORCING_ANALYTIC) {
     out[p] = (T)(c->mag * exy[p]);
     return;
@@ -135,22 +127,30 @@ static int nearest_plane(const solar_ctx* c, double r) {
 }
 
 template <typename T>
-static int launch_force_field(solar_ctx* c, bool advance) {
+static int launch_force_field(solar_ctx* c) {
   const long long n6 = 6LL * c->g.n * c->g.n;
-  const ForceFieldArgs<T> a = {(ForceClock*)c->force_clock, c->forcing, c->force_exy, c->force_samples, n6, (T*)c->force_xy,
-                               c->desc.dt, advance ? 1 : 0};
+  const ForceFieldArgs<T> a = {(const ForceClock*)c->force_clock, c->forcing, c->force_exy, c->force_samples, n6,
+                               (T*)c->force_xy};
   CK(launch_pdl(force_field_kernel<T>, dim3((unsigned)((n6 + 255) / 256)), dim3(256), 0, c->stream, a));
   return SOLAR_OK;
 }
 
-// The source field of the current step; `advance`: the step is taken (the operators leave the
-// clock as it is).
-static int force_begin(solar_ctx* c, bool advance) {
+// The source field of the current step.
+static int force_begin(solar_ctx* c) {
   if (!c->forcing) return SOLAR_OK;
   const ForceClockArgs a = {(ForceClock*)c->force_clock, c->forcing, 695.9894e8, c->ht.dimc, c->desc.dt, c->force_cad,
                             c->force_nstep, c->force_nt, c->err};
   CK(launch_pdl(force_clock_kernel, dim3(1), dim3(1), 0, c->stream, a));
-  return c->fp32 ? launch_force_field<float>(c, advance) : launch_force_field<double>(c, advance);
+  return c->fp32 ? launch_force_field<float>(c) : launch_force_field<double>(c);
+}
+
+// The words that the last kernel of a step advances (a kernel of its own after the filter cost 3 us
+// a step); none without a source.
+static void force_end(const solar_ctx* c, double** time, int** step) {
+  if (!c->forcing) return;
+  ForceClock* const k = (ForceClock*)c->force_clock;      // device addresses
+  *time = &k->time;
+  *step = &k->step;
 }
 
 template <typename T>

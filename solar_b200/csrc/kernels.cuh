@@ -867,6 +867,9 @@ struct FilterArgs {
   Geom g;
   int whole;                // CTAs 0 .. whole-1 filter one (tile, field, face, run) unit each
   int chunks;               // later CTAs filter one of `chunks` radial chunks of a unit
+  double* time;             // the source's clock, advanced by the kernel that ends a step
+  int* step;                // (timestep.f90:82); nullptr in an operator call or without a source
+  double dt;
 };
 
 template <typename T, int TX, int TY>
@@ -939,6 +942,10 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 
   const bool loads = !a.wc.no_loads;
   if (tid == 0 && loads)
     for (int k = ks; k < min(ks + kFiltRing, ke); ++k) issue(k, k - ks);
+  if (a.time && blockIdx.x == 0 && tid == 0) {
+    *a.time = *a.time + a.dt;
+    *a.step = *a.step + 1;
+  }
   T* out = a.qout + g.vol(run, face, s) + g.at(0, j0 + rb, i0 + V * cx);
   constexpr T f0 = T(kFilt[0]), f1 = T(kFilt[1]), f2 = T(kFilt[2]), f3 = T(kFilt[3]);
   constexpr T rw[6] = {T(kFiltR[0]), T(kFiltR[1]), T(kFiltR[2]), T(kFiltR[3]), T(kFiltR[4]), T(kFiltR[5])};

@@ -655,15 +655,19 @@ static long long split_units(long long units, long long nk, int nsm, int residen
   return *whole + (units - *whole) * *chunks_out;
 }
 
+static void force_end(const solar_ctx* c, double** time, int** step);   // forcing.cuh: the clock a step's end advances
+
 template <typename T, int TX, int TY, int R>
-static int launch_filter_t(solar_ctx* c, const void* qin, void* qout, const int* runs) {
+static int launch_filter_t(solar_ctx* c, const void* qin, void* qout, const int* runs, bool step) {
   using L = FilterLayout<T, TX, TY>;
-  FilterArgs<T> a;
+  FilterArgs<T> a = {};
   if (!make_map(c, qin, TX + 8, TY + 6, &a.mP)) return fail(SOLAR_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   a.qout = (T*)qout;
   a.runs = runs;
   a.wc = wait_ctl(c, kInjFilter);
   a.g = c->g;
+  if (step) force_end(c, &a.time, &a.step);
+  a.dt = c->desc.dt;
   static bool attr_set = false;
   static int resident = 1;
   const int threads = (TX / Vec16<T>::V) * (TY / R);
@@ -679,18 +683,19 @@ static int launch_filter_t(solar_ctx* c, const void* qin, void* qout, const int*
   return SOLAR_OK;
 }
 
+// `step`: the launch ends a time step (else FILTER_EXP alone).
 template <typename T>
-static int launch_filter(solar_ctx* c, const void* qin, void* qout, const int* runs) {
+static int launch_filter(solar_ctx* c, const void* qin, void* qout, const int* runs, bool step) {
   // Rows per thread: float keeps one row per thread (four warps of 91 registers, five CTAs
   // to an SM); double takes two, which reads 6 rows of shared memory for 2 output rows
   // (measured at 6 x 128^3: float 100 us with R = 1, 114-119 us with R = 2; double 250 us
   // with R = 2, 282 us with R = 1).
   constexpr int R = sizeof(T) == 4 ? 1 : 2;
-  if (c->g.n % 32 == 0) return launch_filter_t<T, 32, 16, R>(c, qin, qout, runs);
-  return launch_filter_t<T, 16, 16, R>(c, qin, qout, runs);
+  if (c->g.n % 32 == 0) return launch_filter_t<T, 32, 16, R>(c, qin, qout, runs, step);
+  return launch_filter_t<T, 16, 16, R>(c, qin, qout, runs, step);
 }
 
-static int force_begin(solar_ctx* c, bool advance);   // forcing.cuh: this step's source field, its clock
+static int force_begin(solar_ctx* c);   // forcing.cuh: this step's source field
 
 // One full time step (timestep.f90:61-82) on every run.  With ev != nullptr each kernel
 // is bracketed by events: ev_pairs[kind] accumulates into times[kind].
@@ -698,7 +703,7 @@ template <typename T>
 static int enqueue_step(solar_ctx* c, const int* runs, std::vector<cudaEvent_t>* evs) {
   void* bufs[2] = {c->A, c->B};
   int cur = 0, rc;
-  if ((rc = force_begin(c, true))) return rc;
+  if ((rc = force_begin(c))) return rc;
   auto mark = [&]() {
     if (!evs) return;
     cudaEvent_t e;
@@ -717,7 +722,7 @@ static int enqueue_step(solar_ctx* c, const int* runs, std::vector<cudaEvent_t>*
   mark();
   if ((rc = launch_edge<T>(c, bufs[cur], 1, runs))) return rc;
   mark();
-  if ((rc = launch_filter<T>(c, bufs[cur], bufs[cur ^ 1], runs))) return rc;
+  if ((rc = launch_filter<T>(c, bufs[cur], bufs[cur ^ 1], runs, true))) return rc;
   mark();
   return SOLAR_OK;
 }
@@ -1393,7 +1398,7 @@ int solar_gpu_compute_rhs(solar_ctx* c, const double* q, double* rhs) {
   if (rc) return rc;
   if (!q || !rhs) return fail(SOLAR_ERR_ARG, "null array");
   if ((rc = op_prepare_state(c, q))) return rc;
-  if ((rc = force_begin(c, false))) return rc;
+  if ((rc = force_begin(c))) return rc;
   if (c->fp32) { launch_edge<float>(c, c->B, 0, nullptr); rc = launch_stage<float>(c, c->B, c->W, 2, 0, nullptr); }
   else { launch_edge<double>(c, c->B, 0, nullptr); rc = launch_stage<double>(c, c->B, c->W, 2, 0, nullptr); }
   if (rc) return rc;
@@ -1424,8 +1429,8 @@ int solar_gpu_filter_exp(solar_ctx* c, const double* q, double* qf) {
   if (rc) return rc;
   if (!q || !qf) return fail(SOLAR_ERR_ARG, "null array");
   if ((rc = op_prepare_state(c, q))) return rc;
-  if (c->fp32) { launch_edge<float>(c, c->B, 1, nullptr); rc = launch_filter<float>(c, c->B, c->W, nullptr); }
-  else { launch_edge<double>(c, c->B, 1, nullptr); rc = launch_filter<double>(c, c->B, c->W, nullptr); }
+  if (c->fp32) { launch_edge<float>(c, c->B, 1, nullptr); rc = launch_filter<float>(c, c->B, c->W, nullptr, false); }
+  else { launch_edge<double>(c, c->B, 1, nullptr); rc = launch_filter<double>(c, c->B, c->W, nullptr, false); }
   if (rc) return rc;
   CK(cudaGetLastError());
   if ((rc = check_device_error(c))) return rc;

@@ -61,7 +61,7 @@ static int lines_op(solar_ctx* c, int phase, const int* zone_edge, int count, vo
 template <typename T>
 static int enqueue_phase(solar_ctx* c, int phase) {
   int rc;
-  if (phase == 0 && (rc = force_begin(c, true))) return rc;
+  if (phase == 0 && (rc = force_begin(c))) return rc;
   if (phase < 5) {
     void* in = phase % 2 ? c->B : c->A;
     void* out = phase % 2 ? c->A : c->B;
@@ -70,7 +70,7 @@ static int enqueue_phase(solar_ctx* c, int phase) {
   }
   if (phase != 7 && (rc = launch_edge<T>(c, c->B, 1, nullptr))) return rc;
   if (phase == 6) return SOLAR_OK;
-  return launch_filter<T>(c, c->B, c->A, nullptr);
+  return launch_filter<T>(c, c->B, c->A, nullptr, true);
 }
 
 // Phases 0..4 in two parts, so that a process can overlap the edge-line exchange with
@@ -86,7 +86,7 @@ static int enqueue_phase_part(solar_ctx* c, int phase, int part) {
   void* out = phase % 2 ? c->A : c->B;
   const int mode = phase == 0 ? 1 : 0;
   if (part == 0) {
-    if (phase == 0 && (rc = force_begin(c, true))) return rc;
+    if (phase == 0 && (rc = force_begin(c))) return rc;
     return launch_stage<T>(c, in, out, mode, phase, nullptr, nullptr, kTilesInterior);
   }
   if ((rc = launch_edge<T>(c, in, 0, nullptr))) return rc;
