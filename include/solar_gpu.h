@@ -181,7 +181,8 @@ int solar_gpu_set_watchdog(solar_ctx* c, int every);
 #define SOLAR_KERNEL_EDGE 1
 #define SOLAR_KERNEL_STAGE 2
 #define SOLAR_KERNEL_FILTER 4
-#define SOLAR_KERNEL_ADJ_STAGE 8
+#define SOLAR_KERNEL_ADJ_STAGE 8    /* the transposed stage kernel */
+#define SOLAR_KERNEL_ADJ_FILTER 16  /* the transposed filter kernel */
 int solar_gpu_inject_wait_timeout(solar_ctx* c, int kernels, int polls);
 
 /* FP64 diagnostics of one run: out[0] = acoustic energy

@@ -29,6 +29,7 @@ SOLAR_KERNEL_EDGE = 1
 SOLAR_KERNEL_STAGE = 2
 SOLAR_KERNEL_FILTER = 4
 SOLAR_KERNEL_ADJ_STAGE = 8
+SOLAR_KERNEL_ADJ_FILTER = 16
 
 
 class SolarError(RuntimeError):

@@ -774,7 +774,7 @@ __global__ void __launch_bounds__((TX / Vec16<T>::V) * (TY / R), sizeof(T) == 4 
       if (k >= ke) break;
       if (k == ke - release_planes(ke - ks)) release_dependents();
       {
-        const bool got = mbar_wait(&bars[slot], phase, a.wc, kErrAdjointRing);
+        const bool got = mbar_wait(&bars[slot], phase, a.wc, kErrAdjointFilter);
         const T* bx = reinterpret_cast<const T*>(smem + slot * L::P_BYTES);
         T* t1 = reinterpret_cast<T*>(smem + kFiltRing * L::P_BYTES + (k & 1) * L::S_BYTES);
         T c[R + 6][V];                                 // c[m] holds xi-filtered box row rb + m

@@ -156,7 +156,7 @@ static int launch_adj_filter(solar_ctx* c) {
   if (!make_interior_map(c, b.L, TX + 8, TY + 6, &a.mP)) return fail(SOLAR_ERR_CUDA, "cuTensorMapEncodeTiled failed");
   a.qout = (T*)b.T1;
   a.runs = nullptr;
-  a.wc = wait_ctl(c, kInjAdjStage);
+  a.wc = wait_ctl(c, kInjAdjFilter);
   a.g = g;
   constexpr int threads = (TX / Vec16<T>::V) * (TY / R);
   static bool attr_set = false;

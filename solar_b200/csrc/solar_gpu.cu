@@ -26,7 +26,7 @@
 namespace solar {
 
 static_assert(SOLAR_KERNEL_EDGE == kInjEdge && SOLAR_KERNEL_STAGE == kInjStage && SOLAR_KERNEL_FILTER == kInjFilter &&
-                  SOLAR_KERNEL_ADJ_STAGE == kInjAdjStage,
+                  SOLAR_KERNEL_ADJ_STAGE == kInjAdjStage && SOLAR_KERNEL_ADJ_FILTER == kInjAdjFilter,
               "C-ABI kernel bits and device injection bits agree");
 
 thread_local std::string g_last_error;
@@ -738,6 +738,7 @@ static const char* device_error_name(int code) {
     case kErrFilterRing: return "filter kernel";
     case kErrEdgeRing: return "edge kernel";
     case kErrAdjointRing: return "transposed stage kernel";
+    case kErrAdjointFilter: return "transposed filter kernel";
     default: return "unknown kernel";
   }
 }
@@ -1602,7 +1603,7 @@ int solar_gpu_set_watchdog(solar_ctx* c, int every) {
 int solar_gpu_inject_wait_timeout(solar_ctx* c, int kernels, int polls) {
   int rc = check_ctx(c);
   if (rc) return rc;
-  if (kernels & ~(SOLAR_KERNEL_EDGE | SOLAR_KERNEL_STAGE | SOLAR_KERNEL_FILTER | SOLAR_KERNEL_ADJ_STAGE))
+  if (kernels & ~(SOLAR_KERNEL_EDGE | SOLAR_KERNEL_STAGE | SOLAR_KERNEL_FILTER | SOLAR_KERNEL_ADJ_STAGE | SOLAR_KERNEL_ADJ_FILTER))
     return fail(SOLAR_ERR_ARG, "unknown kernel bits 0x%x", kernels);
   if (kernels && (polls < 1 || polls > (int)kWaitPolls)) return fail(SOLAR_ERR_ARG, "polls must be in 1..%u", kWaitPolls);
   CK(cudaStreamSynchronize(c->stream));

@@ -29,11 +29,12 @@ enum DeviceError : int {
   kErrFilterRing = 3,       // filter kernel: ring wait gave up
   kErrEdgeRing = 4,         // edge kernel: ring wait gave up
   kErrAdjointRing = 5,      // transposed stage kernel: ring wait gave up
+  kErrAdjointFilter = 6,    // transposed filter kernel: ring wait gave up
   kErrForcingSample = 16,   // a forcing time sample outside the loaded samples was needed
 };
 
 // Kernels that take part in failure-injection tests (solar_gpu_inject_wait_timeout).
-enum InjectKernel : int { kInjEdge = 1, kInjStage = 2, kInjFilter = 4, kInjAdjStage = 8 };
+enum InjectKernel : int { kInjEdge = 1, kInjStage = 2, kInjFilter = 4, kInjAdjStage = 8, kInjAdjFilter = 16 };
 
 // Wait control carried in a kernel's arguments: the device error word, the bound of one
 // wait in polls, and the injection switch of failure-detection tests (nonzero: the
