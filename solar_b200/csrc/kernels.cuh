@@ -1202,14 +1202,21 @@ __global__ void gaussian_kernel(double* p, Geom g, int face, const double* tanx,
 // writes one partial; the CTA that arrives last adds the partials in a fixed order.  It is part
 // of the step graph, behind the filter kernel (100 steps with norms at 6 x 32^3 in double, state
 // in and out: as two kernels after each replay of the graph 10.18 ms, now 9.75).
+// What a sum is of and where it goes stays in device memory, so that one captured graph serves
+// every field, run and result array.
+struct NormCtl {
+  double* out;              // the sum of this launch goes to out[count] ...
+  long long offset;         // run and slot: values from the volume of (0, face, 0)
+  int arrived;              // CTAs that have arrived (0 between launches)
+  int count;                // ... launches since the host wrote this
+};
+
 template <typename T>
 struct SumsqArgs {
   const T* q;
   double* part;             // [owned faces x planes]
-  double* out;              // out[ctl[1]], ctl[1] counted up by every launch (0 with a single result)
-  int* ctl;                 // [0] CTAs that have arrived (0 between launches), [1] results so far
+  NormCtl* ctl;
   Geom g;
-  int run, slot;
 };
 
 template <typename T>
@@ -1220,8 +1227,8 @@ __global__ void __launch_bounds__(256) sumsq_kernel(const __grid_constant__ Sums
   const int face = g.face0 + blockIdx.x / nk, k = g.k0 + blockIdx.x % nk;
   const int n = g.n, per_row = n / V;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
-  const T* base = a.q + g.vol(a.run, face, a.slot) + g.at(k, 0, 0);
   grid_dependency_wait();
+  const T* base = a.q + a.ctl->offset + g.vol(0, face, 0) + g.at(k, 0, 0);
   double acc = 0.0;
   for (int j = warp; j < n; j += nwarp) {
     const T* row = base + (long long)j * g.pitch;
@@ -1243,7 +1250,7 @@ __global__ void __launch_bounds__(256) sumsq_kernel(const __grid_constant__ Sums
     for (int w = 0; w < nwarp; ++w) t += red[w];
     __stcg(a.part + blockIdx.x, t);
     __threadfence();
-    last = atomicAdd(a.ctl, 1) == (int)gridDim.x - 1;
+    last = atomicAdd(&a.ctl->arrived, 1) == (int)gridDim.x - 1;
   }
   __syncthreads();
   if (!last) return;
@@ -1257,9 +1264,9 @@ __global__ void __launch_bounds__(256) sumsq_kernel(const __grid_constant__ Sums
     __syncthreads();
   }
   if (tid == 0) {
-    a.out[a.ctl[1]] = red[0];
-    a.ctl[0] = 0;
-    a.ctl[1] += 1;
+    a.ctl->out[a.ctl->count] = red[0];
+    a.ctl->arrived = 0;
+    a.ctl->count += 1;
   }
 }
 

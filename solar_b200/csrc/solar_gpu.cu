@@ -194,13 +194,12 @@ struct solar_ctx {
   long long steps_done = 0;    // steps taken by this context (watchdog step numbers)
   double* norm_ring = nullptr; // per-step sums of squares (solar_gpu_rk4_norms)
   int norm_ring_len = 0;
-  int* norm_ctl = nullptr;     // SumsqArgs::ctl
+  NormCtl* norm_ctl = nullptr;
   DevTables dt;
   int tile_x = 32, tile_y = 8, kchunk = 0;
   int edge_resident = 0;       // edge-kernel CTAs per SM (threads and shared memory depend on nx)
   cudaGraphExec_t step_graph = nullptr;
-  cudaGraphExec_t norm_graph = nullptr;   // a step and the sum of squares of one field ...
-  int norm_run = 0, norm_slot = 0;        // ... of this run and slot, into norm_ring
+  cudaGraphExec_t norm_graph = nullptr;   // a step and the sum of squares that norm_ctl names
   std::vector<cudaGraphExec_t> batch_graphs;   // batched step graph per number of live runs
   cudaEvent_t ev[8] = {};
   // FP32 contexts upload the state across PCIe as float: two pinned blocks of one compact
@@ -777,29 +776,33 @@ static int watch_after_step(solar_ctx* c) {
   return SOLAR_OK;
 }
 
-// Sum of squares of one stored field of the state into out[ctl[1]].
+// The sums of the following launches: of one stored field of one run, into out[0], out[1], ...
+static int set_norm(solar_ctx* c, int run, int slot, double* out) {
+  const NormCtl h = {out, c->g.vol(run, 0, slot) - c->g.vol(0, 0, 0), 0, 0};
+  CK(cudaMemcpyAsync(c->norm_ctl, &h, sizeof h, cudaMemcpyHostToDevice, c->stream));
+  return SOLAR_OK;
+}
+
+// Sum of squares of one stored field of the state, as set_norm says.
 template <typename T>
-static int launch_sumsq(solar_ctx* c, int run, int slot, double* out) {
-  const SumsqArgs<T> a = {(const T*)c->A, c->part, out, c->norm_ctl, c->g, run, slot};
+static int launch_sumsq(solar_ctx* c) {
+  const SumsqArgs<T> a = {(const T*)c->A, c->part, c->norm_ctl, c->g};
   CK(launch_pdl(sumsq_kernel<T>, dim3((unsigned)(c->g.nface * (c->g.k1 - c->g.k0))), dim3(256), 0, c->stream, a));
   return SOLAR_OK;
 }
 
-// The step and the norm's sum of one run and slot (slot < 0: the step alone).
-static int capture_norm_graph(solar_ctx* c, int run, int slot) {
-  if (c->norm_graph && c->norm_run == run && c->norm_slot == slot) return SOLAR_OK;
-  if (c->norm_graph) { cudaGraphExecDestroy(c->norm_graph); c->norm_graph = nullptr; }
+// The step and the norm's sum.
+static int capture_norm_graph(solar_ctx* c) {
+  if (c->norm_graph) return SOLAR_OK;
   cudaGraph_t graph;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   int rc = enqueue_step_any(c, nullptr, nullptr);
-  if (!rc && slot >= 0) rc = c->fp32 ? launch_sumsq<float>(c, run, slot, c->norm_ring) : launch_sumsq<double>(c, run, slot, c->norm_ring);
+  if (!rc) rc = c->fp32 ? launch_sumsq<float>(c) : launch_sumsq<double>(c);
   cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
   if (rc) return rc;
   CK(ce);
   CK(cudaGraphInstantiate(&c->norm_graph, graph, 0));
   CK(cudaGraphDestroy(graph));
-  c->norm_run = run;
-  c->norm_slot = slot;
   return SOLAR_OK;
 }
 
@@ -1114,8 +1117,8 @@ static int reduce(solar_ctx* c, int run, int sel_field, double* out5) {
 static int sumsq(solar_ctx* c, int run, int sel_field, double* out) {
   const int s = c->g.slot[sel_field];
   if (s < 0) { *out = 0.0; return SOLAR_OK; }
-  CK(cudaMemsetAsync(c->norm_ctl, 0, 2 * sizeof(int), c->stream));
-  int rc = c->fp32 ? launch_sumsq<float>(c, run, s, c->red_out) : launch_sumsq<double>(c, run, s, c->red_out);
+  int rc = set_norm(c, run, s, c->red_out);
+  if (!rc) rc = c->fp32 ? launch_sumsq<float>(c) : launch_sumsq<double>(c);
   if (rc) return rc;
   CK(cudaMemcpyAsync(out, c->red_out, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
@@ -1252,8 +1255,7 @@ int solar_gpu_init(const solar_desc* d, solar_ctx** out) {
   TRYC(cudaMalloc((void**)&c->stage64, (size_t)vol_compact(c) * sizeof(double)));
   TRYC(cudaMalloc((void**)&c->part, (size_t)6 * g.nr * 5 * sizeof(double)));
   TRYC(cudaMalloc((void**)&c->red_out, 5 * sizeof(double)));
-  TRYC(cudaMalloc((void**)&c->norm_ctl, 2 * sizeof(int)));
-  TRYC(cudaMemset(c->norm_ctl, 0, 2 * sizeof(int)));
+  TRYC(cudaMalloc((void**)&c->norm_ctl, sizeof(NormCtl)));
   TRYC(cudaMalloc((void**)&c->run_order, g.nruns * sizeof(int)));
   TRY(upload_constants());
   if (c->fp32) TRY(upload_tables<float>(c));
@@ -1568,7 +1570,6 @@ int solar_gpu_rk4_norms(solar_ctx* c, int run, int field, int nsteps, double* no
   if (nsteps == 0) return SOLAR_OK;
   if (c->norm_ring_len < nsteps) {
     CK(cudaStreamSynchronize(c->stream));
-    if (c->norm_graph) { cudaGraphExecDestroy(c->norm_graph); c->norm_graph = nullptr; }   // holds the old address
     if (c->norm_ring) cudaFree(c->norm_ring);
     c->norm_ring = nullptr;
     c->norm_ring_len = 0;
@@ -1577,11 +1578,14 @@ int solar_gpu_rk4_norms(solar_ctx* c, int run, int field, int nsteps, double* no
     c->norm_ring_len = nsteps;
   }
   const int slot = c->g.slot[field - 1];
-  if ((rc = capture_norm_graph(c, run, slot))) return rc;
-  CK(cudaMemsetAsync(c->norm_ctl, 0, 2 * sizeof(int), c->stream));
-  if (slot < 0) CK(cudaMemsetAsync(c->norm_ring, 0, (size_t)nsteps * sizeof(double), c->stream));
+  if (slot < 0) {                      // a field the context does not store: norm 0
+    if ((rc = capture_step_graph(c))) return rc;
+    CK(cudaMemsetAsync(c->norm_ring, 0, (size_t)nsteps * sizeof(double), c->stream));
+  } else if ((rc = capture_norm_graph(c)) || (rc = set_norm(c, run, slot, c->norm_ring))) {
+    return rc;
+  }
   for (int s = 0; s < nsteps; ++s) {
-    CK(cudaGraphLaunch(c->norm_graph, c->stream));
+    CK(cudaGraphLaunch(slot < 0 ? c->step_graph : c->norm_graph, c->stream));
     if ((rc = watch_after_step(c))) return rc;
   }
   CK(cudaMemcpyAsync(norms, c->norm_ring, (size_t)nsteps * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
