@@ -31,12 +31,18 @@ static_assert(SOLAR_KERNEL_EDGE == kInjEdge && SOLAR_KERNEL_STAGE == kInjStage &
 
 thread_local std::string g_last_error;
 
-// Host threads of one context for the FP32 state uploads: run(f) calls f(t) for t = 0 ..
-// size()-1, t = 0 on the calling thread, and returns when every call has returned.
+// Host threads of one context for the FP32 state uploads and the staged transfers: run(f) calls
+// f(t) for t = 0 .. size()-1, t = 0 on the calling thread, and returns when every call has
+// returned.  A system that gives fewer threads than asked for makes a smaller pool.
 class HostPool {
  public:
-  explicit HostPool(int n) : n_(std::max(1, n)) {
-    for (int t = 1; t < n_; ++t) th_.emplace_back([this, t] { loop(t); });
+  explicit HostPool(int n) {
+    th_.reserve((size_t)std::max(0, n - 1));
+    try {
+      for (int t = 1; t < n; ++t) th_.emplace_back([this, t] { loop(t); });
+    } catch (const std::exception&) {                 // the threads that did start are kept
+    }
+    n_ = 1 + (int)th_.size();
   }
   ~HostPool() {
     {
@@ -78,7 +84,7 @@ class HostPool {
       if (--left_ == 0) done_.notify_one();
     }
   }
-  int n_;
+  int n_ = 1;
   std::vector<std::thread> th_;
   std::mutex m_;
   std::condition_variable cv_, done_;

@@ -1,0 +1,50 @@
+"""What the transfers do when the host runs short: threads that cannot be started make a smaller
+pool, and a set-up that failed leaves nothing half done.  Each case is a process of its own with
+tests/host_faults.cpp preloaded; nothing fails on the GPU."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+COMMON = """
+import ctypes, sys
+import numpy as np
+from solar_b200 import _lib, configs
+from solar_b200.solver import Solver
+faults = ctypes.CDLL(None)
+def fault(name, value, kind=ctypes.c_int):
+    kind.in_dll(faults, name).value = value
+cfg = configs.c2(nx=64, nr=64)
+q = np.random.default_rng(0).standard_normal((6, 5, 64, 64, 64)).astype(np.float32).astype(np.float64)
+"""
+
+
+@pytest.fixture(scope="module")
+def preload(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("faults") / "host_faults.so")
+    subprocess.check_call(["/usr/bin/g++", "-O1", "-fPIC", "-shared", "-o", so, os.path.join(HERE, "host_faults.cpp"), "-ldl"])
+    return so
+
+
+def run(preload, body):
+    env = dict(os.environ, LD_PRELOAD=preload, PYTHONPATH=os.path.dirname(HERE), OMP_NUM_THREADS="1", OPENBLAS_NUM_THREADS="1")
+    p = subprocess.run([sys.executable, "-c", COMMON + body], env=env, capture_output=True, text=True, timeout=120)
+    assert p.returncode == 0, (p.returncode, p.stderr[-2000:])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("threads", [0, 2])
+def test_few_threads_can_be_started(preload, precision, threads):
+    run(preload, f"""
+with Solver(cfg, precision="{precision}") as s:
+    s.norm(4)
+    fault("threads_left", {threads})
+    s.set_state(q)
+    got = s.get_state()
+    fault("threads_left", -1)
+    np.testing.assert_array_equal(got, q)
+""")
