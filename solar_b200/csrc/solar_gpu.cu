@@ -867,13 +867,18 @@ static int ensure_pool(solar_ctx* c) {
   return SOLAR_OK;
 }
 
-// FP32 transfers: the pinned blocks, their events and the host threads, on first use.
+// FP32 transfers: the host threads, the events and the pinned blocks, on first use.  The blocks
+// come last: they say that all is there.
 static int ensure_pin32(solar_ctx* c) {
   if (c->pin32) return SOLAR_OK;
-  const size_t bytes = (size_t)2 * vol_compact(c) * sizeof(float);
-  CK(cudaHostAlloc((void**)&c->pin32, bytes, cudaHostAllocDefault));
-  for (auto& e : c->xev) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  return ensure_pool(c);
+  int rc;
+  if ((rc = ensure_pool(c))) return rc;
+  for (auto& e : c->xev)
+    if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  void* p = nullptr;
+  CK(cudaHostAlloc(&p, (size_t)2 * vol_compact(c) * sizeof(float), cudaHostAllocDefault));
+  c->pin32 = (float*)p;
+  return SOLAR_OK;
 }
 
 // The slice [lo, hi) of n items that host thread t of p handles.

@@ -48,3 +48,21 @@ with Solver(cfg, precision="{precision}") as s:
     fault("threads_left", -1)
     np.testing.assert_array_equal(got, q)
 """)
+
+
+def test_float_upload_after_a_failed_first_one(preload):
+    """The first upload cannot allocate its pool: an error, and the next upload sets everything up."""
+    run(preload, """
+with Solver(cfg, precision="fp32") as s:
+    s.norm(4)
+    fault("fail_new_min", 120, ctypes.c_size_t)     # the pool: a mutex and two condition variables
+    fault("fail_new_max", 400, ctypes.c_size_t)
+    fault("fail_new", 1)
+    try:
+        s.set_state(q)
+        raise AssertionError("the allocation did not fail")
+    except _lib.SolarError as e:
+        assert e.status == _lib.SOLAR_ERR_NOMEM, e
+    s.set_state(q)
+    np.testing.assert_array_equal(s.get_state(), q)
+""")
