@@ -903,6 +903,9 @@ static int ensure_stage(solar_ctx* c) {
   }
   char* p = (char*)(((uintptr_t)c->pin_map + kStageBytes - 1) / kStageBytes * kStageBytes);
   madvise(p, kStageBlocks * kStageBytes, MADV_HUGEPAGE);      // a hint: small pages work as well
+  // A child process must not share the pages: after a fork, the first write to a shared block could
+  // give this process a new page while the device still reads the old one.
+  if (madvise(p, kStageBlocks * kStageBytes, MADV_DONTFORK)) return fail(SOLAR_ERR_NOMEM, "staging blocks: madvise failed");
   c->pool->run([&](int t) {
     for (int b = t; b < kStageBlocks; b += c->pool->size()) std::memset(p + b * kStageBytes, 0, kStageBytes);
   });

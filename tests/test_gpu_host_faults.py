@@ -66,3 +66,28 @@ with Solver(cfg, precision="fp32") as s:
     s.set_state(q)
     np.testing.assert_array_equal(s.get_state(), q)
 """)
+
+
+def test_staging_blocks_stay_with_the_process(preload):
+    """The pinned blocks (the one mapping with huge pages asked for that appears with the first
+    pageable transfer) are left out of a fork."""
+    run(preload, """
+def advised():
+    found, name = set(), None
+    for line in open("/proc/self/smaps"):
+        first = line.split()[0]
+        if "-" in first and not first.endswith(":"):
+            name = first
+        elif first == "VmFlags:" and "hg" in line.split():
+            found.add((name, "dc" in line.split()))
+    return found
+
+out = np.empty_like(q)
+with Solver(cfg) as s:
+    s.norm(4)
+    before = {name for name, _ in advised()}
+    s.set_state(q)
+    s.set_state(q)
+    new = {(name, kept) for name, kept in advised() if name not in before}
+    assert new and all(kept for _, kept in new), new
+""")
