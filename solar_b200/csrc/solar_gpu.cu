@@ -216,6 +216,7 @@ struct solar_ctx {
   std::unique_ptr<HostPool> pool;
   // Pageable arrays of the caller move through kStageBlocks pinned blocks (on first use).
   char* pin_stage = nullptr;   // inside the mapping pin_map
+  bool stage_off = false;      // they could not be had: not tried again
   void* pin_map = nullptr;
   cudaEvent_t sev[kStageBlocks] = {};
   AdjBuffers adj;
@@ -925,8 +926,12 @@ static bool stage_pageable(solar_ctx* c, const void* p, size_t bytes) {
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return false; }
   if (at.type != cudaMemoryTypeUnregistered) return false;
+  if (c->stage_off) return false;
   if (ensure_stage(c) == SOLAR_OK) return true;
   cudaGetLastError();                                    // no pinned memory or threads: copy as it is
+  c->stage_off = true;
+  if (c->pin_map) munmap(c->pin_map, kStageMap);
+  c->pin_map = nullptr;
   return false;
 }
 

@@ -91,3 +91,17 @@ with Solver(cfg) as s:
     new = {(name, kept) for name, kept in advised() if name not in before}
     assert new and all(kept for _, kept in new), new
 """)
+
+
+def test_staging_that_cannot_be_set_up_is_tried_once(preload):
+    run(preload, """
+MAP = 9 * 2 << 20                                       # eight blocks of 2 MiB and room to align them
+with Solver(cfg) as s:
+    s.norm(4)
+    fault("fail_mmap", MAP, ctypes.c_size_t)
+    for _ in range(3):
+        s.set_state(q)
+        np.testing.assert_array_equal(s.get_state(), q)
+    fault("fail_mmap", 0, ctypes.c_size_t)
+    assert ctypes.c_int.in_dll(faults, "failed_mmaps").value == 1
+""")
