@@ -356,7 +356,7 @@ static int misfit_gradient_t(solar_ctx* c, int N, int K, int K2, const double* d
   }
   if (grad_c) {
     const size_t bytes = (size_t)V6 * sizeof(double);
-    if (bytes >= 8u << 20 && stage_pageable(c, grad_c, bytes)) {
+    if (bytes >= 8u << 20 && pageable_volumes(grad_c, bytes) && stage_download(c, grad_c, bytes)) {
       Staged st(c);
       if ((rc = st.out(grad_c, b.grad, bytes)) || (rc = st.finish())) return rc;
     } else {

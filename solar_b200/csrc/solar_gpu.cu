@@ -5,6 +5,7 @@
 
 #include <sched.h>
 #include <sys/mman.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <cmath>
@@ -217,6 +218,7 @@ struct solar_ctx {
   // Pageable arrays of the caller move through kStageBlocks pinned blocks (on first use).
   char* pin_stage = nullptr;   // inside the mapping pin_map
   bool stage_off = false;      // they could not be had: not tried again
+  size_t pageable_in = 0;      // bytes uploaded from pageable arrays before the blocks were set up
   void* pin_map = nullptr;
   cudaEvent_t sev[kStageBlocks] = {};
   AdjBuffers adj;
@@ -915,17 +917,16 @@ static int ensure_stage(solar_ctx* c) {
   return SOLAR_OK;
 }
 
-// Whether an array of the caller, moved in volumes of `bytes`, goes through the pinned blocks:
-// pageable memory in volumes of at least 1 MiB.  The driver moves such arrays through a staging
-// buffer of its own with one thread, which also takes the page faults of a fresh result array
-// (COMPUTE_RHS at 6 x 64^3 in double, 63 MB out into fresh memory: 16.2 ms, now 6.3; at 6 x 96^3
-// 50 ms, now 18; a pageable state in at 6 x 96^3 19.4 ms, now 7.0).  Smaller volumes do not
-// repay waking the threads (6 x 48^3, 0.9 MB each: the same 3.2 ms).
-static bool stage_pageable(solar_ctx* c, const void* p, size_t bytes) {
+// Pageable arrays of the caller, moved in volumes of at least 1 MiB, may go through the pinned
+// blocks; smaller volumes do not repay waking the threads (6 x 48^3, 0.9 MB each: the same 3.2 ms).
+static bool pageable_volumes(const void* p, size_t bytes) {
   if (bytes < (1u << 20)) return false;
   cudaPointerAttributes at;
   if (cudaPointerGetAttributes(&at, p) != cudaSuccess) { cudaGetLastError(); return false; }
-  if (at.type != cudaMemoryTypeUnregistered) return false;
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
+static bool stage_ready(solar_ctx* c) {
   if (c->stage_off) return false;
   if (ensure_stage(c) == SOLAR_OK) return true;
   cudaGetLastError();                                    // no pinned memory or threads: copy as it is
@@ -933,6 +934,34 @@ static bool stage_pageable(solar_ctx* c, const void* p, size_t bytes) {
   if (c->pin_map) munmap(c->pin_map, kStageMap);
   c->pin_map = nullptr;
   return false;
+}
+
+// Whether an upload of `total` bytes from p, in volumes of `bytes`, is staged.  The driver moves
+// pageable arrays through a staging buffer of its own with one thread (a state in at 6 x 96^3 in
+// double 19.2 ms, staged 7.9; at 6 x 48^2 x 58 3.0 and 1.6 ms).  Setting the blocks up takes 2 to 3
+// ms, the gain of about 50 MB, so they are set up when a context has uploaded as much (a first
+// upload of 32 MB at 6 x 48^2 x 58: staged 3.4 .. 5 ms, directly 2.8 .. 3.6).
+constexpr size_t kStageFrom = 48u << 20;
+static bool stage_upload(solar_ctx* c, const void* p, size_t bytes, size_t total) {
+  if (!pageable_volumes(p, bytes)) return false;
+  if (!c->pin_stage && (c->pageable_in += total) < kStageFrom) return false;
+  return stage_ready(c);
+}
+
+// Whether a volume read back to p, in pageable memory, is staged: where its pages are not there yet.
+// The driver's one thread takes their page faults, the host threads share them (a state out into
+// fresh memory at 6 x 64^3 in double 29 ms, staged 5.6; 6 x 128^3 220 and 41 ms).  Into memory that
+// is there the driver is faster (4.5 against 5.3 ms; 30 against 49).  Four pages of the volume are
+// looked at; what the system does not tell counts as there.
+static bool stage_download(solar_ctx* c, void* p, size_t bytes) {
+  static const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+  int there = 0;
+  for (int q = 0; q < 4; ++q) {
+    unsigned char v = 1;
+    const uintptr_t at = ((uintptr_t)p + bytes / 8 * (2 * q + 1)) / page * page;
+    there += mincore((void*)at, page, &v) || (v & 1) ? 1 : 0;
+  }
+  return there < 2 && stage_ready(c);
 }
 
 // Copies between the device and a pageable array, on the context's stream, through the pinned
@@ -1049,7 +1078,7 @@ static int upload_fields(solar_ctx* c, void* buf, int run, const double* host, i
   if (c->fp32) return upload_fields32(c, buf, run, host, nh, fields, nfields_h);
   const long long V = vol_compact(c);
   const size_t bytes = (size_t)V * sizeof(double);
-  const bool staged = stage_pageable(c, host, bytes);
+  const bool staged = stage_upload(c, host, bytes, (size_t)6 * nfields_h * bytes);
   Staged st(c);
   const int threads = 256;
   const int blocks = (int)((V + threads - 1) / threads);
@@ -1077,7 +1106,7 @@ static int download_fields(solar_ctx* c, const void* buf, int run, double* host,
                            const int* fields, int nfields_h) {
   const long long V = vol_compact(c);
   const size_t bytes = (size_t)V * sizeof(double);
-  const bool staged = stage_pageable(c, host, bytes);
+  const bool pageable = pageable_volumes(host, bytes);
   Staged st(c);
   int rc;
   const int threads = 256;
@@ -1094,7 +1123,7 @@ static int download_fields(solar_ctx* c, const void* buf, int run, double* host,
       if (c->fp32) pack_kernel<float><<<blocks, threads, 0, c->stream>>>((const float*)buf + c->g.vol(run, z, s), c->stage64, c->g);
       else pack_kernel<double><<<blocks, threads, 0, c->stream>>>((const double*)buf + c->g.vol(run, z, s), c->stage64, c->g);
       CK(cudaGetLastError());
-      if (staged) {
+      if (pageable && stage_download(c, dst, bytes)) {
         if ((rc = st.out(dst, c->stage64, bytes))) return rc;
       } else {
         CK(cudaMemcpyAsync(dst, c->stage64, bytes, cudaMemcpyDeviceToHost, c->stream));
