@@ -79,7 +79,7 @@ struct AdjStageArgs {
 // What bounds it: the latency of a plane's loads.  Requests count as much as bytes: with one TMA
 // request per field (14 per plane in double) a reverse step at 6 x 96^3 took 2045 us in double and
 // 850 in float, with the fields of one shape in one 4-D request (8 per plane) 1681 and 838.  Two
-// slots keep two CTAs per SM in double (110 KB each) and four in float (51 KB).  The form before
+// slots keep two CTAs per SM in double (110 KB each) and four in float (52 KB).  The form before
 // (one point per thread, lambda_w and lambda_q boxes, two barriers per plane, a kernel of its own
 // for the one-sided rows) took 2163 and 1198.
 constexpr int kAdjRing = 2;
@@ -87,8 +87,8 @@ constexpr int kAdjRing = 2;
 // Rounding.  dt L^T(mu) is small against lambda_q, so its terms are summed up before lambda_q comes
 // in wherever registers allow, and what has to be added to the large sum later is added in as few
 // parts as possible.  Error of lambda after 1 / 20 reverse steps in float against double, 6 x 48^2 x
-// 33, 6 x 96^3: 1.12e-7 / 2.84e-7, 1.20e-7 / 3.23e-7; with lambda_q first and every plane's radial
-// term added to it by itself 1.53e-7 / 3.42e-7, 1.65e-7 / 4.15e-7.  In float lambda_q of p, v_xi and
+// 33 and 6 x 96^3: 1.12e-7 / 2.84e-7 and 1.20e-7 / 3.23e-7; with lambda_q first and every plane's radial
+// term added to it by itself 1.53e-7 / 3.42e-7 and 1.65e-7 / 4.15e-7.  In float lambda_q of p, v_xi and
 // v_eta waits for the terms behind the barrier, and a plane's radial term of p for the next plane's
 // (a step takes 0.3% less with four fields, 2.6% less with five, mean over ten grids from 6 x 64^3
 // to 6 x 128^3).  In double the registers are used up: the same costs 5-30%, so there lambda_q
@@ -696,7 +696,7 @@ __global__ void adj_edge_kernel(const __grid_constant__ AdjEdgeArgs<T> a) {
 // filter, being last, is followed by none that smooths it (error in float 4.8e-8; centre first
 // 8.4e-8, with the radial filter first and the xi filter last 7.5e-8; the same time).  Tiles,
 // threads, ring and work split are those of filter_kernel, and so is what bounds it.  us per
-// launch at 6 x 96^3 in double / float: 116 / 54, with adj_ghost_kernel's 42 / 29 beside it (as a
+// launch at 6 x 96^3 in double / float: 117 / 55, and adj_ghost_kernel 42 / 29 after it (as a
 // radial pass over the whole buffer and a plane-marching xi/eta pass with plain loads, ghost
 // adjoints included, 117 + 170 / 52 + 67; with a branch around the zero planes 134 / 69).
 template <typename T, int TX, int TY, int R>

@@ -889,7 +889,7 @@ struct FilterLayout {
 // rows above and the 3 below its own, eta-filters its R x V points and pushes them into an
 // 11-deep register queue; the k loop is unrolled by 11 so the queue indices are constants.
 // With R = 2 a thread reads 6 rows from shared memory for 2 output rows instead of 7 for 1.
-// The float kernel's bound of four CTAs per SM lets the compiler use 91 registers: at 6 x
+// The float kernel's bound of four CTAs per SM lets the compiler use 93 registers: at 6 x
 // 128^3 it ran in 100 us against 106 us at 88 registers (a bound of five) and 115 us at 83
 // (no bound).  The filter weights are compile-time values (scheme.h).
 template <typename T, int TX, int TY, int R>

@@ -694,7 +694,7 @@ static int launch_filter_t(solar_ctx* c, const void* qin, void* qout, const int*
 // `step`: the launch ends a time step (else FILTER_EXP alone).
 template <typename T>
 static int launch_filter(solar_ctx* c, const void* qin, void* qout, const int* runs, bool step) {
-  // Rows per thread: float keeps one row per thread (four warps of 91 registers, five CTAs
+  // Rows per thread: float keeps one row per thread (four warps of 93 registers, five CTAs
   // to an SM); double takes two, which reads 6 rows of shared memory for 2 output rows
   // (measured at 6 x 128^3: float 100 us with R = 1, 114-119 us with R = 2; double 250 us
   // with R = 2, 282 us with R = 1).

@@ -1,5 +1,5 @@
 """Host arrays of every kind the transfers tell apart: pageable and pinned, volumes below 1 MiB
-(copied as they are), above it (through the pinned blocks) and above one 4 MiB block with a
+(copied as they are), above it (through the pinned blocks) and above one 2 MiB block with a
 remainder.  Transfers move values, so FP64 results are equal bit for bit."""
 import numpy as np
 import pytest
